@@ -46,6 +46,32 @@ def test_row_bands_and_strided_out(kind):
     assert (big[:, n:] == -7.0).all()  # nothing written past the row
 
 
+@pytest.mark.parametrize("dt", ["float32", "float64"])
+@pytest.mark.parametrize("n,lead,shift,rb,re", [
+    (63, 0, 0, 0, 63), (64, 0, 1, 0, 64), (65, 3, 5, 0, 65), (97, 0, 31, 3, 90), (129, 31, 0, 64, 129),
+    (1024, 0, 0, 0, 1024), (1024, 1, 0, 0, 1024), (4501, 0, 3, 0, 4501), (4501, 0, 0, 1000, 1100),
+    (4160, 32, 0, 0, 4160), (13001, 0, 0, 0, 13001), (13056, 0, 8, 6000, 13056)])
+def test_expansion_strips_and_tiles(n, lead, shift, rb, re, dt):
+    """Whole-line tiles and column strips: row starts on and inside 128-byte
+    lines (`lead` elements between rows, `shift` before the first), one and
+    several segments, row bands; nothing outside the band's rows is written."""
+    import torch
+    dt = getattr(torch, dt)
+    for kind, diagonal in (("distance", -1), ("symmetric", 0)):
+        i, j = torch.tril_indices(n, n, diagonal, device="cuda")
+        st = torch.rand(i.numel(), device="cuda", dtype=dt)
+        want = torch.zeros((n, n), device="cuda", dtype=dt)
+        want[i, j] = st
+        want[j, i] = st
+        del i, j
+        buf = torch.full((shift + (re - rb) * (n + lead) + 64,), -7.0, device="cuda", dtype=dt)
+        rows = buf[shift:shift + (re - rb) * (n + lead)].view(re - rb, n + lead)
+        dev.condensed_to_dense(st, n, kind, rb, re, out=rows[:, :n])
+        assert torch.equal(rows[:, :n], want[rb:re])
+        assert bool((rows[:, n:] == -7.0).all()) and bool((buf[:shift] == -7.0).all())
+        assert bool((buf[shift + rows.numel():] == -7.0).all())
+
+
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 @pytest.mark.parametrize("kind", ["distance", "symmetric"])
 def test_dense_to_condensed_round_trip(dt, kind):
