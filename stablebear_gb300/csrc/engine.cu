@@ -12,6 +12,7 @@
 //     overlaps the kernel of band b + 1.
 #include "sbg_internal.hpp"
 #include "host_copy.hpp"
+#include "fixed_point.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -619,7 +620,7 @@ namespace sbg
   // of one problem.  The queue counter is stream-ordered scratch.
   template <typename T>
   static void launch_problem(ProblemDesc<T> d, const Plan& pl, int opk, cudaStream_t st,
-                             unsigned long long* given_queue = nullptr)
+                             unsigned long long* given_queue = nullptr, const unsigned* gate = nullptr)
   {
     d.item_begin = 0;
     d.n_items = problem_item_count(d);
@@ -631,7 +632,7 @@ namespace sbg
       own.reset(new AsyncBuf<T>(sizeof(unsigned long long), st));
       queue = static_cast<unsigned long long*>(own->p);
     }
-    SBG_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
+    if (!gate) SBG_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));  // else zeroed with the gate's own
     LaunchParams<T> L{};
     L.one = d;
     L.probs = nullptr;
@@ -642,8 +643,129 @@ namespace sbg
     L.row_cap = pl.row_cap;
     L.win_r = pl.win_r;
     L.row_slots = pl.row_slots;
+    L.gate = gate;
     const int grid = (int)std::min<uint64_t>((uint64_t)pl.grid, d.n_items);
     SBG_CUDA(launch_pairs<T>(L, opk, pl.kvar, pl.warps, grid, pl.smem_bytes, st));
+  }
+
+  // ---- double precision in fixed point (fixed_point.cu) ---------------------------
+
+  namespace
+  {
+    // One call's fixed-point run: the record of its data, the packed arrays
+    // and the launches, in one device buffer.  The direct kernel of the plan
+    // is launched behind every fixed one, gated by the record.
+    struct FixedRun
+    {
+      int opk = 0, sms = 0;
+      uint32_t q = 1, smem = 0;
+      uint64_t rcap = 0, ccap = 0;
+      bool cross = false;
+      bool used[2] = {false, false};  // whose queue counters are no longer zero
+      char* base = nullptr;
+      size_t rpack = 0, rshape = 0, rlens = 0, cpack = 0, cshape = 0, clens = 0, carry = 0, carry_bytes = 0, total = 0;
+
+      static constexpr size_t GATE = 128, QUEUES = 192;  // the record at 0
+      static constexpr int SLOTS = 2;                    // launches in flight (one per stream)
+
+      // Queue counters of the fixed and the gated direct launch.
+      unsigned long long* queue(int slot) const { return reinterpret_cast<unsigned long long*>(base + QUEUES) + 2 * slot; }
+      FixedRecord* record() const { return reinterpret_cast<FixedRecord*>(base); }
+      unsigned* gate() const { return reinterpret_cast<unsigned*>(base + GATE); }
+      void* rows() const { return base + rpack; }
+      void* cols() const { return cross ? base + cpack : base + rpack; }
+      uint32_t* row_lens() const { return reinterpret_cast<uint32_t*>(base + rlens); }
+      uint32_t* col_lens() const { return reinterpret_cast<uint32_t*>(base + (cross ? clens : rlens)); }
+      Shape* row_shapes() const { return reinterpret_cast<Shape*>(base + rshape); }
+      Shape* col_shapes() const { return reinterpret_cast<Shape*>(base + (cross ? cshape : rshape)); }
+
+      // Whether a call takes this path: every automatic one, whatever its
+      // size (30 PCFs of L ~ U{16..200}, L1 on the device: 116 us a call
+      // against 304 with the direct kernel, whose chain of FP64 latencies
+      // alone is longer than all the launches here).
+      static bool wanted(int opk)
+      {
+        if (settings().variant.load() != 0 || settings().windowCap.load() != 0) return false;
+        return opk == OPK_L1 || opk == OPK_L2DIST || opk == OPK_INNER;
+      }
+      void layout(int opk_, int mode, uint64_t nr, uint64_t nc, uint32_t lmax, uint64_t row_points, uint64_t col_points,
+                  uint64_t row_begin, const DeviceInfo& dev, int slots)
+      {
+        opk = opk_;
+        sms = dev.sms;
+        cross = mode == MODE_CROSS;
+        rcap = std::max<uint64_t>(row_points, 1);
+        ccap = cross ? std::max<uint64_t>(col_points, 1) : rcap;
+        q = 1;
+        for (uint32_t cand : {4u, 2u})
+          if (row_begin % (32 * cand) == 0 && items_for(mode, 0, nr, nc, cand) >= (uint64_t)dev.sms * 6)
+          {
+            q = cand;
+            break;
+          }
+        smem = (uint32_t)(dev.smem_optin - 2048);
+        auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+        rpack = 256;
+        rshape = rpack + up(rcap * 16);
+        rlens = rshape + up(nr * sizeof(Shape));
+        cpack = rlens + up(nr * sizeof(uint32_t));
+        cshape = cpack + up(ccap * 16);
+        clens = cshape + up(nc * sizeof(Shape));
+        carry = cross ? clens + up(nc * sizeof(uint32_t)) : cpack;
+        // one window takes every PCF, in the larger of the two element sizes
+        const uint32_t slots_bytes = (32 * q * 4 + 15) / 16 * 16;
+        const bool one = lmax <= fixed_slice_cap(smem - slots_bytes, FIXED_WARPS, 16);
+        carry_bytes = one ? 0 : up((size_t)sms * 32 * q * FIXED_CARRY * 32 * 8);
+        total = carry + slots * carry_bytes;
+      }
+      // The record and the packed arrays (elements for the direct kernel
+      // where the record asks for it and that kernel reads them).
+      // rperm / cperm: where the processing order by packed lengths goes, or
+      // null.
+      void prepare(char* at, const PcfSet<double>& r, const PcfSet<double>& c, bool elements, uint32_t* rperm,
+                   uint32_t* cperm, cudaStream_t st)
+      {
+        base = at;
+        SBG_CUDA(cudaMemsetAsync(base, 0, 256, st));
+        SBG_CUDA(launch_fixed_record(r.pts, r.off, r.n, rcap, record(), sms, st));
+        if (cross) SBG_CUDA(launch_fixed_record(c.pts, c.off, c.n, ccap, record(), sms, st));
+        SBG_CUDA(launch_fixed_pack(r.pts, r.off, r.n, rcap, record(), opk, rows(), row_shapes(), row_lens(), elements, gate(), sms, st));
+        if (cross) SBG_CUDA(launch_fixed_pack(c.pts, c.off, c.n, ccap, record(), opk, cols(), col_shapes(), col_lens(), elements, gate(), sms, st));
+        if (rperm) length_order_device(r.off, r.n, rperm, nullptr, st, row_lens());
+        if (cross && cperm) length_order_device(c.off, c.n, cperm, nullptr, st, col_lens());
+      }
+      // One launch over the rows and output of `d` (points: the callers' CSR),
+      // and the direct kernel behind it.
+      void launch(ProblemDesc<double> d, const double* rpts, const double* cpts, const Plan& pl, int slot,
+                  cudaStream_t st)
+      {
+        FixedParams P{};
+        P.rec = record();
+        P.r = FixedSet{rpts, d.roff, d.rperm, d.nr, static_cast<const uint64_t*>(rows()), rcap, row_shapes(), row_lens()};
+        P.c = FixedSet{cpts, d.coff, d.cperm, d.nc, static_cast<const uint64_t*>(cols()), ccap, col_shapes(), col_lens()};
+        P.out = d.out; P.out_base = d.out_base; P.out_count = d.out_count; P.ld = d.ld;
+        P.row_begin = d.row_begin; P.row_end = d.row_end;
+        P.mode = d.mode;
+        P.q = q;
+        P.rows_per_item = 32 * q;
+        P.smem_bytes = smem;
+        P.carry = reinterpret_cast<uint64_t*>(base + carry + (size_t)slot * carry_bytes);
+        P.n_items = items_for(d.mode, d.row_begin, d.row_end, d.nc, q);
+        if (P.n_items == 0) return;
+        P.queue = queue(slot);
+        if (used[slot]) SBG_CUDA(cudaMemsetAsync(P.queue, 0, 2 * sizeof(unsigned long long), st));
+        used[slot] = true;
+        SBG_CUDA(launch_fixed_pairs(P, opk, (int)std::min<uint64_t>(P.n_items, (uint64_t)sms), st));
+        if (pl.packed)
+        {
+          d.rpts = static_cast<const double*>(rows());
+          d.cpts = static_cast<const double*>(cols());
+          d.rcap = rcap;
+          d.ccap = ccap;
+        }
+        launch_problem<double>(d, pl, opk, st, queue(slot) + 1, gate());
+      }
+    };
   }
 
   template <typename T>
@@ -679,6 +801,7 @@ namespace sbg
     // contiguous output range.  The permutation is the one the host entry
     // uses, so both give the same bits.
     std::unique_ptr<AsyncBuf<T>> order_buf;
+    size_t order_perm_bytes = 0;
     const bool windows = row_begin % LENGTH_ORDER_WINDOW == 0 &&
                          (row_end % LENGTH_ORDER_WINDOW == 0 || row_end == rows.n);
     const bool caller_perm = rperm || cperm;
@@ -686,19 +809,19 @@ namespace sbg
         cs.n <= 0xffffffffull)
     {
       const uint64_t nr = rows.n, nc = (mode == MODE_CROSS) ? cs.n : 0;
-      const size_t perm_bytes = ((nr + nc) * sizeof(uint32_t) + 255) / 256 * 256;
+      const size_t perm_bytes = order_perm_bytes = ((nr + nc) * sizeof(uint32_t) + 255) / 256 * 256;
       const size_t key_bytes = std::max(length_order_scratch_bytes(nr), length_order_scratch_bytes(nc));
       order_buf.reset(new AsyncBuf<T>(perm_bytes + key_bytes, st));
       uint32_t* rp = static_cast<uint32_t*>(order_buf->p);
-      void* keys = static_cast<char*>(order_buf->p) + perm_bytes;
-      length_order_device(rows.off, nr, rp, keys, st);
       rperm = rp;
-      if (mode == MODE_CROSS)
-      {
-        length_order_device(cs.off, nc, rp + nr, keys, st);
-        cperm = rp + nr;
-      }
+      if (mode == MODE_CROSS) cperm = rp + nr;
     }
+    auto order_by_points = [&] {
+      if (!order_buf) return;
+      void* keys = static_cast<char*>(order_buf->p) + order_perm_bytes;
+      length_order_device(rows.off, rows.n, const_cast<uint32_t*>(rperm), keys, st);
+      if (mode == MODE_CROSS) length_order_device(cs.off, cs.n, const_cast<uint32_t*>(cperm), keys, st);
+    };
 
     ProblemDesc<T> d{};
     d.rpts = rows.pts; d.roff = rows.off; d.rperm = rperm; d.nr = rows.n;
@@ -714,16 +837,45 @@ namespace sbg
       d.out_count = hi > out_base ? hi - out_base : 0;
     }
 
-    // Packed segment layout for the global-memory variant (needs the point
-    // totals, read back with one synchronisation).
-    std::unique_ptr<AsyncBuf<T>> rpack, cpack;
+    // Packed layouts need the point totals: read back with one
+    // synchronisation for the global-memory and hybrid variants; the
+    // fixed-point path of a call that needs none otherwise sizes its buffer
+    // for PCFs of the longest length.
+    uint64_t rtot = 0, ctot = 0;
     if (pl.packed)
     {
-      uint64_t rtot = 0, ctot = 0;
       SBG_CUDA(cudaMemcpyAsync(&rtot, rows.off + rows.n, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
       if (mode == MODE_CROSS)
         SBG_CUDA(cudaMemcpyAsync(&ctot, cs.off + cs.n, sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
       SBG_CUDA(cudaStreamSynchronize(st));
+    }
+    if constexpr (sizeof(T) == 8)
+    {
+      if (FixedRun::wanted(opk))
+      {
+        FixedRun run;
+        run.layout(opk, mode, rows.n, cs.n, lmax, pl.packed ? rtot : rows.n * lmax, pl.packed ? ctot : cs.n * lmax,
+                   row_begin, dev, 1);
+        std::unique_ptr<AsyncBuf<T>> buf;
+        try { buf.reset(new AsyncBuf<T>(run.total, st)); }
+        catch (const Error& e)
+        {
+          if (e.status != ST_OUT_OF_MEMORY) throw;  // the direct path needs less
+        }
+        if (buf)
+        {
+          run.prepare(static_cast<char*>(buf->p), rows, cs, pl.packed,
+                      order_buf ? const_cast<uint32_t*>(rperm) : nullptr,
+                      order_buf ? const_cast<uint32_t*>(cperm) : nullptr, st);
+          run.launch(d, rows.pts, cs.pts, pl, 0, st);
+          return;
+        }
+      }
+    }
+    order_by_points();
+    std::unique_ptr<AsyncBuf<T>> rpack, cpack;
+    if (pl.packed)
+    {
       rpack.reset(new AsyncBuf<T>(sizeof(Elem<T>) * std::max<uint64_t>(rtot, 1), st));
       SBG_CUDA(launch_pack<T>(rows.pts, rows.off, rows.n, (Elem<T>*)rpack->p, rtot, dev.sms, st));
       d.rpts = reinterpret_cast<const T*>(rpack->p);
@@ -1040,11 +1192,32 @@ namespace sbg
     EventGuard computed[2], copied[2];
     phases.mark("buffers");
 
-    // Packed segment layout, once, for the global-memory variant.
-    DeviceBuffer rpack, cpack;
+    // Packed segment layout, once, for the global-memory variant; or the
+    // fixed-point path's arrays.
+    DeviceBuffer rpack, cpack, fixed_buf;
     const T* kr_pts = drows.view.pts;
     const T* kc_pts = (mode == MODE_CROSS) ? dcols.view.pts : drows.view.pts;
-    if (pl.packed)
+    FixedRun fixed;
+    if constexpr (sizeof(T) == 8)
+    {
+      const int k = op_kind(op, p);
+      if (FixedRun::wanted(k))
+      {
+        fixed.layout(k, mode, rows.n, cs.n, lmax, rows.off[rows.n], cs.off[cs.n], 0, dev, FixedRun::SLOTS);
+        try { fixed_buf.reset(fixed.total); }
+        catch (const Error& e)
+        {
+          if (e.status != ST_OUT_OF_MEMORY) throw;  // the direct path needs less
+        }
+        if (fixed_buf.get())
+        {
+          fixed.prepare(fixed_buf.as<char>(), drows.view, mode == MODE_CROSS ? dcols.view : drows.view, pl.packed,
+                        sorted ? drperm.as<uint32_t>() : nullptr,
+                        sorted && mode == MODE_CROSS ? dcperm.as<uint32_t>() : nullptr, compute.s);
+        }
+      }
+    }
+    if (pl.packed && !fixed_buf.get())
     {
       rpack.reset(sizeof(Elem<T>) * std::max<uint64_t>(1, rows.off[rows.n]));
       SBG_CUDA(launch_pack<T>(drows.view.pts, drows.view.off, rows.n, rpack.as<Elem<T>>(), rows.off[rows.n], dev.sms,
@@ -1095,6 +1268,15 @@ namespace sbg
       // it.  No pair's arithmetic depends on the item shape.
       if (!direct)
         while (d.q % 2 == 0 && problem_item_count(d) < 6ull * (uint64_t)dev.sms) d.q /= 2;
+      if constexpr (sizeof(T) == 8)
+      {
+        if (fixed_buf.get())
+        {
+          fixed.launch(d, drows.view.pts, mode == MODE_CROSS ? dcols.view.pts : drows.view.pts, pl, b, bs);
+          SBG_CUDA(cudaEventRecord(computed[b].e, bs));
+          return;
+        }
+      }
       launch_problem<T>(d, pl, opk, bs);
       SBG_CUDA(cudaEventRecord(computed[b].e, bs));
     };

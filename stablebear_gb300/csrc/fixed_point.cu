@@ -1,0 +1,925 @@
+// Pairwise integrals of float64 PCFs in 64-bit fixed point (sm_103a).
+//
+// The FP64 pipe of this GPU retires about two lanes per SM and clock, 1/64 of
+// the FP32 rate, and the merge of pair_kernels.cu needs three to four FP64
+// operations per rectangle: 58 to 78 SM cycles per warp-step, all spent on
+// that pipe.  Here the merge runs on the integer pipe.  Times become integers
+// T = rint(t 2^s) below 2^62, values integers too, and
+//   sum over rectangles of (T_right - T_left) * op(F, G)
+// is an exact integer sum: it does not depend on the order of the pair, the
+// processing order, window ends or the launch shape.  FP64 appears once per
+// pair, where the sum becomes a double.
+//
+// Values come in two forms, chosen on the device from the data:
+//   counts   every value a multiple of one power of two with at most 13 bits
+//            (26 for L1), as the ranks and Betti numbers of persistence
+//            summaries are.  op(F, G) is an exact 32-bit integer; a rectangle
+//            costs two 32 x 32 -> 64 multiply-adds (times are kept as two
+//            31-bit limbs whose differences need no carry).
+//   general  |F| < 2^62; op(F, G) is the top 64 bits of the product, times
+//            the 62-bit width into a 128-bit sum.
+//
+// Error.  A time is off by at most half a unit, so a sum is off by at most
+// half the total change of op(F, G) along the merge, which the two PCFs'
+// variations bound; general values add at most two units of op per unit of
+// time.
+// A pair whose bound is above 2^-47 of the sum of |terms| (the worst case of
+// the direct walk's naive blocks of 64) is walked again in double precision,
+// as is every pair of a call whose data fits no form (NaN or infinite values,
+// times out of order, extreme exponents or outliers): then pairs_kernel or
+// the hybrid kernel runs instead, gated by the same device-side record.
+#include "sbg_internal.hpp"
+
+#include "fixed_point.cuh"
+
+namespace sbg
+{
+  namespace
+  {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int U = 8;                                  // steps per block
+    constexpr uint64_t T_END = (1ull << 62) - 1;          // after every breakpoint
+    constexpr int MAX_EXP = 300;                          // larger exponents go the direct way
+    constexpr uint32_t LOW_BIAS = 4096;
+
+    // ---- the record of the data ---------------------------------------------------
+
+    __device__ __forceinline__ int exponent(double x)  // of a finite x > 0: 2^e <= x < 2^(e + 1)
+    {
+      const uint64_t b = (uint64_t)__double_as_longlong(x);
+      const int e = (int)(b >> 52) & 0x7ff;
+      return e ? e - 1023 : 63 - __clzll((long long)(b & 0xfffffffffffffull)) - 1074;
+    }
+    __device__ __forceinline__ int low_exponent(double x)  // of the lowest set bit of a finite x != 0
+    {
+      const uint64_t b = (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull;
+      const int e = (int)(b >> 52);
+      const uint64_t m = (b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
+      return (e ? e : 1) - 1075 + __ffsll((long long)m) - 1;
+    }
+    __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+
+    // What the record says: the form and its scales.
+    struct Form
+    {
+      int kind;   // 0 direct, 1 counts, 2 general
+      int s;      // T = rint(t 2^s)
+      int r;      // F = rint(v 2^r)
+      bool sign;  // some value is negative
+    };
+
+    __device__ Form form_of(const FixedRecord& d, int opk)
+    {
+      Form f{0, 0, 0, d.negative != 0};
+      if (d.bad) return f;
+      const double tmax = __longlong_as_double((long long)d.tmax_bits);
+      const double vmax = __longlong_as_double((long long)d.vmax_bits);
+      int te = 0, ve = 0, low = 0;
+      if (tmax > 0) te = exponent(tmax);
+      if (vmax > 0)
+      {
+        ve = exponent(vmax);
+        low = (int)LOW_BIAS - (int)d.low;
+      }
+      if (te > MAX_EXP || te < -MAX_EXP || ve > MAX_EXP || low < -MAX_EXP) return f;
+      f.s = 61 - te;
+      if (ve - low < (opk == OPK_L1 ? 26 : 13))
+      {
+        f.kind = 1;
+        f.r = -low;
+        return f;
+      }
+      // Outliers push the other values down to the general form's last
+      // bits, and its pairs to the direct walk: such data goes there at once.
+      const double mean = d.vsum / (double)(d.points ? d.points : 1);
+      if (mean < vmax * (opk == OPK_L1 ? 0x1p-11 : 0x1p-6)) return f;
+      f.kind = 2;
+      f.r = 61 - ve;
+      return f;
+    }
+
+    // One warp per PCF.  Times count from the second breakpoint on (the walk
+    // starts at 0 whatever the first says).
+    __global__ void __launch_bounds__(256) fixed_record_kernel(const double* __restrict__ pts,
+                                                               const uint64_t* __restrict__ off, uint64_t n,
+                                                               uint64_t cap, FixedRecord* rec)
+    {
+      const int lane = threadIdx.x & 31;
+      const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+      const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+      // the largest time and |value| as bit patterns; NaN and inf order above every finite one
+      uint64_t tmax = 0, vmax = 0;
+      uint32_t low = 0, neg = 0, bad = 0;
+      float vsum = 0.0f;
+      uint64_t points = 0;
+      constexpr uint64_t INF = 0x7ff0000000000000ull;
+      for (uint64_t i = w; i < n; i += nw)
+      {
+        const uint64_t o = off[i], e = off[i + 1];
+        if (e <= o || e > cap || e - o > 0xffffffffull) { bad = 1; continue; }
+        const uint64_t len = e - o;
+        points += lane == 0 ? len : 0;
+        for (uint64_t k = lane; k < len; k += 32)
+        {
+          const double t = pts[2 * (o + k)], v = pts[2 * (o + k) + 1];  // 8-byte aligned, no more
+          if (k > 0)
+          {
+            const uint64_t tb = (uint64_t)__double_as_longlong(t);
+            // times >= 0 order as their bit patterns; a set sign bit is above them all
+            const uint64_t before = k > 1 ? (uint64_t)__double_as_longlong(pts[2 * (o + k - 1)]) : 0;
+            bad |= tb < before || tb >= INF ? 1u : 0u;
+            if (v != pts[2 * (o + k) - 1]) tmax = tb > tmax ? tb : tmax;  // no breakpoint of the function otherwise
+          }
+          const uint64_t vb = (uint64_t)__double_as_longlong(v) & 0x7fffffffffffffffull;
+          if (vb)
+          {
+            vmax = vb > vmax ? vb : vmax;
+            neg |= __double_as_longlong(v) < 0 ? 1u : 0u;
+            const uint32_t l = (uint32_t)((int)LOW_BIAS - low_exponent(v));
+            low = l > low ? l : low;
+            vsum += fabsf((float)v);
+          }
+        }
+      }
+      if (vmax >= INF) bad = 1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+      {
+        const uint64_t a = __shfl_xor_sync(FULL, tmax, o), b = __shfl_xor_sync(FULL, vmax, o);
+        tmax = a > tmax ? a : tmax;
+        vmax = b > vmax ? b : vmax;
+        vsum += __shfl_xor_sync(FULL, vsum, o);
+      }
+      low = __reduce_max_sync(FULL, low);
+      neg = __reduce_or_sync(FULL, neg);
+      bad = __reduce_or_sync(FULL, bad);
+      if (lane == 0)
+      {
+        if (bad) atomicOr(&rec->bad, 1u);
+        if (neg) atomicOr(&rec->negative, 1u);
+        atomicMax(&rec->low, low);
+        atomicMax(reinterpret_cast<unsigned long long*>(&rec->tmax_bits), (unsigned long long)tmax);
+        atomicMax(reinterpret_cast<unsigned long long*>(&rec->vmax_bits), (unsigned long long)vmax);
+        atomicAdd(&rec->vsum, (double)vsum);
+        atomicAdd(reinterpret_cast<unsigned long long*>(&rec->points), (unsigned long long)points);
+      }
+    }
+
+    // The times of a PCF's elements (an element ends where the value next
+    // changes, the last at T_END) and their values, at the CSR's own offsets,
+    // and how many there are: neighbours of equal value are one element (a
+    // rank that has reached 0 and stays there, say), which changes no exact
+    // sum.  Where the record says direct, the (v, t) elements the hybrid
+    // kernel reads, in the same buffer, all of them.  One warp per PCF.
+    __global__ void __launch_bounds__(256) fixed_pack_kernel(const double* __restrict__ pts,
+                                                             const uint64_t* __restrict__ off, uint64_t n,
+                                                             uint64_t cap, const FixedRecord* __restrict__ rec, int opk,
+                                                             void* __restrict__ packed, Shape* __restrict__ shapes,
+                                                             uint32_t* __restrict__ lens, bool elements,
+                                                             unsigned* __restrict__ gate)
+    {
+      const Form f = form_of(*rec, opk);
+      if (blockIdx.x == 0 && threadIdx.x == 0) *gate = f.kind == 0 ? 0u : 1u;  // closes the direct kernels
+      const int lane = threadIdx.x & 31;
+      const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+      const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+      uint64_t* times = static_cast<uint64_t*>(packed);
+      void* values = times + cap;
+      const double ts = pow2(f.s), vs = pow2(f.r), unit = pow2(f.kind == 1 ? f.r : f.r - 32);
+      for (uint64_t i = w; i < n; i += nw)
+      {
+        const uint64_t o = off[i], e = off[i + 1];
+        if (e <= o || e > cap)  // never write past the packed buffer
+        {
+          if (lane == 0) lens[i] = 0;
+          continue;
+        }
+        const uint64_t len = e - o;
+        if (f.kind == 0)
+        {
+          if (lane == 0) lens[i] = (uint32_t)len;
+          if (elements)
+            for (uint64_t k = lane; k < len; k += 32)
+              static_cast<Elem<double>*>(packed)[o + k] =
+                  Elem<double>{pts[2 * (o + k) + 1],
+                               k + 1 == len ? tmax_of<double>() : fmin(pts[2 * (o + k + 1)], tmax_of<double>())};
+          continue;
+        }
+        float tv = 0.0f, qv = 0.0f, vm = 0.0f;
+        uint64_t count = 0;  // elements before this chunk
+        for (uint64_t k0 = 0; k0 < len; k0 += 32)
+        {
+          const uint64_t k = k0 + lane;
+          double t = 0.0, v = 0.0, before = 0.0;
+          if (k < len)
+          {
+            t = pts[2 * (o + k)];
+            v = pts[2 * (o + k) + 1];
+            if (k > 0) before = pts[2 * (o + k) - 1];
+          }
+          const bool starts = k < len && (k == 0 || v != before);
+          const unsigned mask = __ballot_sync(FULL, starts);
+          if (starts)
+          {
+            const uint64_t at = o + count + __popc(mask & ((1u << lane) - 1u));  // <= o + k
+            const long long F = __double2ll_rn(v * vs);
+            const float d = k == 0 ? 0.0f : fabsf((float)((v - before) * unit));
+            tv += d;
+            qv += d * d;
+            vm = fmaxf(vm, fabsf((float)F) * (f.kind == 1 ? 1.0f : 0x1p-32f));
+            if (f.kind == 1)
+              static_cast<uint32_t*>(values)[at] = (uint32_t)(int32_t)F;
+            else
+              // the product needs magnitudes and signs, differences need two's complement
+              static_cast<uint64_t*>(values)[at] =
+                  opk == OPK_INNER ? (uint64_t)(F < 0 ? -F : F) | (F < 0 ? 1ull << 63 : 0ull) : (uint64_t)F;
+            if (k > 0)  // ends the element before
+            {
+              const uint64_t T = (uint64_t)__double2ll_rn(t * ts);
+              times[at - 1] = f.kind == 1 ? ((T >> 31) << 32) | (T & 0x7fffffffull) : T;
+            }
+          }
+          count += (uint64_t)__popc(mask);
+        }
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1)
+        {
+          tv += __shfl_xor_sync(FULL, tv, h);
+          qv += __shfl_xor_sync(FULL, qv, h);
+          vm = fmaxf(vm, __shfl_xor_sync(FULL, vm, h));
+        }
+        if (lane == 0)
+        {
+          times[o + count - 1] = f.kind == 1 ? ((T_END >> 31) << 32) | (T_END & 0x7fffffffull) : T_END;
+          lens[i] = (uint32_t)count;
+          shapes[i] = Shape{tv, qv, vm, 0.0f};
+        }
+      }
+    }
+
+    // ---- arithmetic of the two forms -----------------------------------------------
+
+    // Running sums of one lane's pair.
+    //   add      one rectangle: op(F, G) = q, found before its side moved on
+    //   good     whether the error bound is within 2^-47 of the sum of |terms|
+    //   value    the sum as a double, in units of time times op
+    //
+    // Error of the times, in units of op.  Worst case: half the change of op
+    // along the merge, which the PCFs' own variation bounds (Shape), for the
+    // square by Cauchy-Schwarz: with no two breakpoints at once,
+    //   sum |q' - q| = sum |d' - d| |d' + d| <= 2 sqrt(sum (d' - d)^2 sum q).
+    // Or six standard deviations of independent roundings (each 1 / sqrt(12)
+    // of its change of op), where that is less.
+    template <int K>
+    __device__ __forceinline__ float time_error(const Shape& f, const Shape& g, float sum_q)
+    {
+      if (K == OPK_L1) return fminf(0.5f * (f.tv + g.tv), 1.75f * sqrtf(f.qv + g.qv));
+      if (K == OPK_INNER)
+        return fminf(0.5f * (f.vmax * g.tv + g.vmax * f.tv),
+                     1.75f * sqrtf(f.vmax * f.vmax * g.qv + g.vmax * g.vmax * f.qv));
+      return sqrtf(f.qv + g.qv) * sqrtf(sum_q);
+    }
+
+    // Kept as 32-bit registers throughout: as 64-bit C++ variables the walk's
+    // tied asm operands and the products cost ten more instructions a step
+    // (28 against 18 for counts).
+    template <int K, bool SG>
+    struct Counts
+    {
+      using V = uint32_t;
+      struct Side { uint32_t lo, hi, v; };    // where the element ends (two 31-bit limbs), its value
+      struct Q { int32_t q; };
+      static constexpr uint32_t BYTES = 12;   // of an element in shared memory
+      int64_t s0 = 0, s1 = 0;                 // sum = s1 2^31 + s0
+      uint64_t extra = 0;                     // L2: sum of q over the steps; signed products: sum of |q| times the high limb
+      uint32_t qs = 0;
+
+      static __device__ __forceinline__ uint64_t end() { return ((T_END >> 31) << 32) | (T_END & 0x7fffffffull); }
+      static __device__ __forceinline__ Q op(const Side& f, const Side& g)
+      {
+        // in asm: the compiler would widen the product to 64 bits
+        int32_t q;
+        if (K == OPK_INNER) asm("mul.lo.s32 %0, %1, %2;" : "=r"(q) : "r"(f.v), "r"(g.v));
+        else if (K == OPK_L1) asm("abs.s32 %0, %1;" : "=r"(q) : "r"(f.v - g.v));
+        else asm("mul.lo.s32 %0, %1, %1;" : "=r"(q) : "r"(f.v - g.v));
+        return Q{q};
+      }
+      __device__ __forceinline__ void add(uint32_t tl, uint32_t th, uint32_t nl, uint32_t nh, Q q)
+      {
+        const int32_t lo = (int32_t)(nl - tl), hi = (int32_t)(nh - th);
+        s0 += (int64_t)q.q * lo;
+        s1 += (int64_t)q.q * hi;
+        if (K == OPK_L2DIST) qs += (uint32_t)q.q;
+        if (SG) extra += (uint64_t)(uint32_t)abs(q.q) * (uint32_t)hi;
+      }
+      __device__ __forceinline__ void block()  // s0 stays below 2^63 over a block's 8 steps of 2^28 * 2^31
+      {
+        s1 += s0 >> 31;
+        s0 &= 0x7fffffff;
+        if (K == OPK_L2DIST)
+        {
+          extra += qs;
+          qs = 0;
+        }
+      }
+      __device__ __forceinline__ void save(uint64_t* c) const
+      {
+        c[0] = (uint64_t)s0; c[32] = (uint64_t)s1; c[64] = extra;
+      }
+      __device__ __forceinline__ void restore(const uint64_t* c)
+      {
+        s0 = (int64_t)c[0]; s1 = (int64_t)c[32]; extra = c[64];
+      }
+      __device__ __forceinline__ bool good(const Shape& f, const Shape& g, uint64_t) const
+      {
+        const float total = SG ? (float)extra : (float)s1;
+        return time_error<K>(f, g, (float)extra) * 0x1p47f <= total * 0x1p31f;
+      }
+      __device__ __forceinline__ double value() const { return fma((double)s1, 0x1p31, (double)s0); }
+      static __device__ __forceinline__ int scale(const Form& f) { return -f.s - (K == OPK_L1 ? f.r : 2 * f.r); }
+    };
+
+    template <int K, bool SG>
+    struct General
+    {
+      using V = uint64_t;
+      struct Side { uint32_t lo, hi, v, w; };  // where the element ends, its value (low, high word)
+      struct Q { uint32_t lo, hi, sign; };     // |op|, all ones where it is negative
+      static constexpr uint32_t BYTES = 16;
+      uint32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;  // sum = s + h 2^64 + negatives
+      uint64_t h = 0, extra = 0;                // extra: as for Counts, of the high words
+      uint32_t negatives = 0;                   // terms subtracted as their one's complement
+
+      static __device__ __forceinline__ uint64_t end() { return T_END; }
+      static __device__ __forceinline__ Q op(const Side& f, const Side& g)
+      {
+        if (K == OPK_INNER)  // magnitudes and signs: the top word of the product
+        {
+          const uint32_t fw = SG ? f.w & 0x7fffffffu : f.w, gw = SG ? g.w & 0x7fffffffu : g.w;
+          uint64_t r = (((uint64_t)f.v * g.v) >> 32) + (uint64_t)f.v * gw;
+          r += (uint64_t)fw * g.v;
+          const uint64_t q = (r >> 32) + (uint64_t)fw * gw;
+          return Q{(uint32_t)q, (uint32_t)(q >> 32), SG ? (uint32_t)((int32_t)(f.w ^ g.w) >> 31) : 0u};
+        }
+        uint32_t al, ah;
+        asm("{\n\t.reg .b32 s;\n\t"
+            "sub.cc.u32 %0, %2, %4;\n\t"
+            "subc.u32 %1, %3, %5;\n\t"
+            "shr.s32 s, %1, 31;\n\t"
+            "xor.b32 %0, %0, s;\n\t"
+            "xor.b32 %1, %1, s;\n\t"
+            "sub.cc.u32 %0, %0, s;\n\t"
+            "subc.u32 %1, %1, s;\n\t}"
+            : "=&r"(al), "=&r"(ah)
+            : "r"(f.v), "r"(f.w), "r"(g.v), "r"(g.w));
+        if (K == OPK_L1) return Q{al, ah, 0u};
+        const uint64_t r = (((uint64_t)al * al) >> 32) + (uint64_t)al * (ah + ah);  // |d| < 2^63: no carry out
+        const uint64_t q = (r >> 32) + (uint64_t)ah * ah;
+        return Q{(uint32_t)q, (uint32_t)(q >> 32), 0u};
+      }
+      __device__ __forceinline__ void add(uint32_t tl, uint32_t th, uint32_t nl, uint32_t nh, Q q)
+      {
+        uint32_t bl, bh;
+        asm("sub.cc.u32 %0, %2, %4;\n\tsubc.u32 %1, %3, %5;"
+            : "=&r"(bl), "=r"(bh)
+            : "r"(nl), "r"(nh), "r"(tl), "r"(th));
+        const uint64_t p = (uint64_t)q.lo * bl;
+        uint64_t r = (p >> 32) + (uint64_t)q.lo * bh;
+        r += (uint64_t)q.hi * bl;
+        if (SG)
+        {
+          const uint64_t t = (r >> 32) + (uint64_t)q.hi * bh;
+          asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;"
+              : "+r"(s0), "+r"(s1), "+r"(s2), "+r"(s3)
+              : "r"((uint32_t)p ^ q.sign), "r"((uint32_t)r ^ q.sign), "r"((uint32_t)t ^ q.sign),
+                "r"((uint32_t)(t >> 32) ^ q.sign));
+          negatives -= q.sign;
+          extra += (uint64_t)q.hi * bh;
+        }
+        else
+        {
+          h += (uint64_t)q.hi * bh;
+          asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, 0;"
+              : "+r"(s0), "+r"(s1), "+r"(s2), "+r"(s3)
+              : "r"((uint32_t)p), "r"((uint32_t)r), "r"((uint32_t)(r >> 32)));
+        }
+        if (K == OPK_L2DIST) extra += q.hi;
+      }
+      __device__ __forceinline__ void block() { }
+      __device__ __forceinline__ unsigned __int128 sum() const
+      {
+        const unsigned __int128 lo = ((uint64_t)s1 << 32) | s0, hi = (((uint64_t)s3 << 32) | s2) + h;
+        return (hi << 64) + lo + negatives;
+      }
+      __device__ __forceinline__ void save(uint64_t* c) const
+      {
+        const unsigned __int128 s = sum();
+        c[0] = (uint64_t)s; c[32] = (uint64_t)(s >> 64); c[64] = extra;
+      }
+      __device__ __forceinline__ void restore(const uint64_t* c)
+      {
+        s0 = (uint32_t)c[0]; s1 = (uint32_t)(c[0] >> 32);
+        s2 = (uint32_t)c[32]; s3 = (uint32_t)(c[32] >> 32);
+        extra = c[64];
+      }
+      // Shapes are in units of 2^32 here.  Besides the times: the values' own
+      // rounding and the dropped low word, two units of op over the time T of
+      // the later last breakpoint.
+      __device__ __forceinline__ bool good(const Shape& f, const Shape& g, uint64_t T) const
+      {
+        const float total = (float)(SG ? extra : (uint64_t)(sum() >> 64));  // in units of 2^64
+        const float times = time_error<K>(f, g, ((float)extra + 8192.0f) * 0x1p32f) * (K == OPK_L1 ? 0x1p32f : 1.0f);
+        return (times + (float)T * 2.0f) * 0x1p-17f <= total;
+      }
+      __device__ __forceinline__ double value() const
+      {
+        const __int128 s = (__int128)sum();
+        const bool neg = SG && s < 0;
+        const unsigned __int128 a = (unsigned __int128)(neg ? -s : s);
+        const double v = fma((double)(uint64_t)(a >> 64), 0x1p64, (double)(uint64_t)a);
+        return neg ? -v : v;
+      }
+      static __device__ __forceinline__ int scale(const Form& f)
+      {
+        return K == OPK_L1 ? -f.s - f.r : 64 - f.s - 2 * f.r;
+      }
+    };
+
+    // ---- the walk -----------------------------------------------------------------
+
+    // A row of a warp in shared memory: times, then values; a lane's column:
+    // elements 32 BYTES bytes apart.  (nl, nh): the next breakpoint, the row's
+    // on a tie.  One side moves on, with loads for that side alone.
+    template <typename A>
+    __device__ __forceinline__ void advance(typename A::Side& f, typename A::Side& g, uint32_t& af, uint32_t tof,
+                                            uint32_t& ag, uint32_t vof, uint32_t& nl, uint32_t& nh)
+    {
+      if constexpr (sizeof(typename A::V) == 4)
+        // af: address of the row value; its time lies at 2 af + tof
+        asm("{\n\t.reg .pred p;\n\t.reg .b32 a, b;\n\t.reg .u64 x, y;\n\t"
+            "mov.b64 x, {%0, %1};\n\t"
+            "mov.b64 y, {%3, %4};\n\t"
+            "setp.le.u64 p, x, y;\n\t"
+            "selp.b32 %8, %0, %3, p;\n\t"
+            "selp.b32 %9, %1, %4, p;\n\t"
+            "@p add.u32 %6, %6, 4;\n\t"
+            "@!p add.u32 %7, %7, 384;\n\t"
+            "mad.lo.u32 a, %6, 2, %10;\n\t"
+            "add.u32 b, %7, %11;\n\t"
+            "@p ld.shared.v2.u32 {%0, %1}, [a];\n\t"
+            "@p ld.shared.u32 %2, [%6];\n\t"
+            "@!p ld.shared.v2.u32 {%3, %4}, [%7];\n\t"
+            "@!p ld.shared.u32 %5, [b];\n\t}"
+            : "+r"(f.lo), "+r"(f.hi), "+r"(f.v), "+r"(g.lo), "+r"(g.hi), "+r"(g.v), "+r"(af), "+r"(ag), "=&r"(nl),
+              "=&r"(nh)
+            : "r"(tof), "r"(vof));
+      else
+        // af: address of the row value; its time lies at af + tof
+        asm("{\n\t.reg .pred p;\n\t.reg .b32 a;\n\t.reg .u64 x, y;\n\t"
+            "mov.b64 x, {%0, %1};\n\t"
+            "mov.b64 y, {%4, %5};\n\t"
+            "setp.le.u64 p, x, y;\n\t"
+            "selp.b32 %10, %0, %4, p;\n\t"
+            "selp.b32 %11, %1, %5, p;\n\t"
+            "@p add.u32 %8, %8, 8;\n\t"
+            "@!p add.u32 %9, %9, 512;\n\t"
+            "add.u32 a, %8, %12;\n\t"
+            "@p ld.shared.v2.u32 {%0, %1}, [a];\n\t"
+            "@p ld.shared.v2.u32 {%2, %3}, [%8];\n\t"
+            "@!p ld.shared.v4.u32 {%4, %5, %6, %7}, [%9];\n\t}"
+            : "+r"(f.lo), "+r"(f.hi), "+r"(f.v), "+r"(f.w), "+r"(g.lo), "+r"(g.hi), "+r"(g.v), "+r"(g.w), "+r"(af),
+              "+r"(ag), "=&r"(nl), "=&r"(nh)
+            : "r"(tof));
+    }
+
+    // Steps through one (sub-)window: the row's m elements from t0 / v0, the
+    // last ending at the window's end and followed by U copies of itself; the
+    // lane's column from address ag.  Nothing passes the row's end, so a
+    // column that reaches further is cut there.
+    template <typename A>
+    __device__ __forceinline__ void walk(A& acc, const uint64_t* t0, const typename A::V* v0, uint32_t ag,
+                                         uint32_t vof, uint32_t m, uint32_t steps, uint64_t t)
+    {
+      using V = typename A::V;
+      typename A::Side f, g;
+      f.lo = (uint32_t)*t0;
+      f.hi = (uint32_t)(*t0 >> 32);
+      f.v = (uint32_t)*v0;
+      const uint32_t at = (uint32_t)__cvta_generic_to_shared(t0);
+      uint32_t af = (uint32_t)__cvta_generic_to_shared(v0);
+      const uint32_t tof = sizeof(V) == 4 ? at - 2 * af : at - af;
+      const uint32_t af_last = af + (m - 1) * (uint32_t)sizeof(V);
+      if constexpr (sizeof(V) == 4)
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%3];\n\tld.shared.u32 %2, [%4];"
+                     : "=&r"(g.lo), "=&r"(g.hi), "=r"(g.v)
+                     : "r"(ag), "r"(ag + vof)
+                     : "memory");
+      else
+      {
+        f.w = (uint32_t)(*v0 >> 32);
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(g.lo), "=r"(g.hi), "=r"(g.v), "=r"(g.w)
+                     : "r"(ag)
+                     : "memory");
+      }
+      uint32_t tl = (uint32_t)t, th = (uint32_t)(t >> 32);
+      const uint32_t nblk = (steps + U - 1) / U;
+      for (uint32_t b = 0; b < nblk; ++b)
+      {
+        // a lane past its end advances the row on every step: back to the
+        // last element, of which U copies follow
+        af = min(af, af_last);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+          const auto q = A::op(f, g);
+          uint32_t nl, nh;
+          advance<A>(f, g, af, tof, ag, vof, nl, nh);
+          acc.add(tl, th, nl, nh, q);
+          tl = nl;
+          th = nh;
+        }
+        acc.block();
+      }
+    }
+
+    template <int K>
+    __device__ __forceinline__ double op_f64(double f, double g)
+    {
+      const double d = f - g;
+      return K == OPK_INNER ? f * g : K == OPK_L1 ? fabs(d) : d * d;
+    }
+
+    // A pair in double precision, from the CSR points, by the whole warp: the
+    // longer PCF's elements split over the lanes, each lane's part walked in
+    // naive blocks of 64 rectangles under Kahan compensation, as the direct
+    // kernels sum, and the parts added.  (By the pair's own lane, its chain of
+    // dependent loads, one long row after the other, kept one SM busy for 23 ms
+    // at N = 1200: one column whose PCF ends at a very early time fails the
+    // test against every row.)
+    template <int K>
+    __device__ __noinline__ double direct_pair(const double* f, uint32_t nf, const double* g, uint32_t ng)
+    {
+      if (nf < ng)
+      {
+        const double* p = f; f = g; g = p;
+        const uint32_t n = nf; nf = ng; ng = n;
+      }
+      const double TM = tmax_of<double>();
+      const uint32_t lane = threadIdx.x & 31;
+      const uint32_t per = (nf + 31) / 32, first = lane * per, end = min(nf, first + per);
+      double acc = 0.0;
+      if (first < end)
+      {
+        uint32_t i = first, j = 0;
+        double t = i ? f[2 * i] : 0.0;
+        for (uint32_t lo = 1, hi = ng; lo < hi;)  // the first of g's breakpoints after t
+        {
+          const uint32_t mid = (lo + hi) / 2;
+          if (g[2 * mid] <= t) { lo = mid + 1; j = mid; } else hi = mid;
+        }
+        double ft = i + 1 < nf ? f[2 * i + 2] : TM, gt = j + 1 < ng ? g[2 * j + 2] : TM, fv = f[2 * i + 1],
+               gv = g[2 * j + 1], comp = 0.0, blk = 0.0;
+        for (uint32_t k = 1;; ++k)
+        {
+          const double tn = ft <= gt ? ft : gt;
+          if (tn != t) blk = fma(op_f64<K>(fv, gv), tn - t, blk);
+          t = tn;
+          // a lane's part ends with its last element's own breakpoint
+          const bool done = ft <= gt && (i + 1 == end || (ft == TM && gt == TM));
+          if (k % 64 == 0 || done)
+          {
+            const double y = blk - comp, s = acc + y;
+            comp = isfinite(s) ? (s - acc) - y : 0.0;
+            acc = s;
+            blk = 0.0;
+          }
+          if (done) break;
+          if (ft <= gt)
+          {
+            ++i;
+            fv = f[2 * i + 1];
+            ft = i + 1 < nf ? f[2 * i + 2] : TM;
+          }
+          else
+          {
+            ++j;
+            gv = g[2 * j + 1];
+            gt = j + 1 < ng ? g[2 * j + 2] : TM;
+          }
+        }
+        acc -= comp;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
+      return acc;
+    }
+
+    // First k in [lo, hi] whose element of this lane's staged column ends
+    // after x (STRICT) or at or after x; element hi always does.
+    template <bool STRICT>
+    __device__ __forceinline__ uint32_t column_find(const unsigned char* col, uint32_t stride, uint32_t lo, uint32_t hi,
+                                                    uint64_t x)
+    {
+      while (lo < hi)
+      {
+        const uint32_t mid = (lo + hi) >> 1;
+        const uint64_t tn = *reinterpret_cast<const uint64_t*>(col + (size_t)mid * stride);
+        if (STRICT ? tn > x : tn >= x) hi = mid; else lo = mid + 1;
+      }
+      return lo;
+    }
+
+    // Items, time windows and row pieces as in pairs_window_kernel
+    // (pair_kernels.cu): the 32 columns of an item in shared memory, window
+    // by window, each warp walking its rows against them.  A PCF that fits
+    // the block is one window.  Sums pass from window to window through
+    // P.carry, exactly.
+    template <int K, typename A>
+    __device__ void run_items(const FixedParams& P, const Form& form, unsigned char* smem)
+    {
+      using V = typename A::V;
+      constexpr uint32_t EB = A::BYTES, CS = 32 * EB;  // bytes between a column's elements
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+      __shared__ unsigned long long s_item;
+      __shared__ unsigned int s_next_row;
+      __shared__ unsigned long long s_bend;
+      __shared__ uint32_t s_ck0[32], s_cnt[32], s_cm[32];
+
+      uint32_t* rk0 = reinterpret_cast<uint32_t*>(smem);
+      unsigned char* cols = smem + (P.rows_per_item * 4 + 15) / 16 * 16;
+      const uint32_t X = fixed_slice_cap(P.smem_bytes - (P.rows_per_item * 4 + 15) / 16 * 16, (uint32_t)nwarps, EB);
+      const uint32_t RB = fixed_row_elements(X);
+      uint64_t* rt = reinterpret_cast<uint64_t*>(cols + (size_t)X * CS + (size_t)warp * RB * EB);
+      V* rv = reinterpret_cast<V*>(rt + RB);
+      // this lane's column: element k's time at lcol + k CS, its value vof further
+      unsigned char* lcol = cols + (size_t)lane * (sizeof(V) == 4 ? 8 : 16);
+      const uint32_t vof = sizeof(V) == 4 ? 256u - 4u * (uint32_t)lane : 8u;
+      uint64_t* carry = P.carry + (size_t)blockIdx.x * P.rows_per_item * FIXED_CARRY * 32;
+
+      const uint64_t END = A::end();
+      const double unit = pow2(A::scale(form));
+      const V* rvals = reinterpret_cast<const V*>(P.r.times + P.r.cap);
+      const V* cvals = reinterpret_cast<const V*>(P.c.times + P.c.cap);
+      const uint64_t G = ceil_div_u64(P.c.n, 32);
+
+      for (;;)
+      {
+        if (threadIdx.x == 0) s_item = atomicAdd(P.queue, 1ull);
+        __syncthreads();
+        if (s_item >= P.n_items) break;
+        // from the last item down: in length order a window's longest rows
+        // come last, and the longest items are best started first
+        const unsigned long long item = P.n_items - 1 - s_item;
+        uint64_t c, g;
+        if (P.mode == MODE_CROSS) { c = item / G; g = item % G; }
+        else tri_decode(item, P.row_begin, P.row_end, P.q, G, &c, &g);
+        uint64_t row_lo = P.row_begin + c * 32ull * P.q;
+        uint64_t row_hi = row_lo + 32ull * P.q;
+        if (row_hi > P.row_end) row_hi = P.row_end;
+        const uint64_t col0 = 32ull * g;
+        if (P.mode != MODE_CROSS)
+        {
+          const uint64_t first = col0 + (P.mode == MODE_PDIST ? 1 : 0);
+          if (row_lo < first) row_lo = first;
+        }
+        const uint32_t nrows = row_hi > row_lo ? (uint32_t)(row_hi - row_lo) : 0u;
+
+        // this lane's column; lanes past the last one mirror lane 0's
+        const uint64_t cj = col0 + lane;
+        const bool cvalid = cj < P.c.n;
+        uint64_t corig = P.c.perm ? P.c.perm[cvalid ? cj : col0] : (cvalid ? cj : col0);
+        const bool pgood = corig < P.c.n;
+        if (!pgood) corig = 0;
+        const uint64_t coff = P.c.off[corig];
+        const uint32_t cpoints = (uint32_t)(P.c.off[corig + 1] - coff);  // >= 1 (the record)
+        const uint32_t clen = P.c.lens[corig];                           // 1 to cpoints, inside the packed arrays
+        const uint64_t* ctime = P.c.times + coff;
+        const V* cval = cvals + coff;
+        const double clast = P.c.pts[2 * (coff + cpoints) - 1];
+        const Shape cshape = P.c.shapes[corig];
+
+        if (nrows > 0 && nrows <= P.rows_per_item)
+        {
+          for (uint32_t r = threadIdx.x; r < nrows; r += blockDim.x) rk0[r] = 0;
+          if (threadIdx.x < 32) s_ck0[threadIdx.x] = 0;
+          uint64_t Ab = 0;  // the window is [Ab, Be)
+          bool first = true;
+          for (;;)
+          {
+            if (threadIdx.x < 32) s_cnt[threadIdx.x] = 0;
+            if (threadIdx.x == 0) s_next_row = 0;
+            if (warp == 0)
+            {
+              // the window ends with the earliest X-th element of a column,
+              // counted from its first element ending after Ab
+              uint32_t k0 = s_ck0[lane];
+              while (k0 + 1 < clen && ctime[k0] <= Ab) ++k0;
+              s_ck0[lane] = k0;
+              uint64_t b = (uint64_t)k0 + X < clen ? ctime[k0 + X - 1] : END;
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1)
+              {
+                const uint64_t y = __shfl_xor_sync(FULL, b, o);
+                b = y < b ? y : b;
+              }
+              if (lane == 0) s_bend = b;
+            }
+            __syncthreads();
+            const uint64_t Be = s_bend;
+            const bool last = Be >= END;
+
+            // column slices, cut at the window's end
+            {
+              const uint32_t k0 = s_ck0[lane];
+              const uint32_t avail = min(X, clen - k0);
+              uint32_t cnt = 0;
+              for (uint32_t k = warp; k < avail; k += nwarps)
+              {
+                const uint64_t tn = ctime[k0 + k];
+                cnt += tn < Be ? 1u : 0u;
+                *reinterpret_cast<uint64_t*>(lcol + (size_t)k * CS) = tn < Be ? tn : Be;
+                *reinterpret_cast<V*>(lcol + (size_t)k * CS + vof) = cval[k0 + k];
+              }
+              if (cnt) atomicAdd(&s_cnt[lane], cnt);
+            }
+            __syncthreads();
+            if (warp == 0)
+            {
+              const uint32_t k0 = s_ck0[lane];
+              const uint32_t m = min(s_cnt[lane] + 1u, min(X, clen - k0));
+              s_cm[lane] = m;
+              s_ck0[lane] = k0 + m - 1;  // reaches the window's end
+            }
+            __syncthreads();
+            const uint32_t cm = s_cm[lane];
+            const uint32_t maxmc = __reduce_max_sync(FULL, cm);
+
+            for (;;)
+            {
+              unsigned r = 0;
+              if (lane == 0) r = atomicAdd(&s_next_row, 1u);
+              r = __shfl_sync(FULL, r, 0);
+              if (r >= nrows) break;
+              const uint64_t i = row_lo + r;
+              const uint64_t iorig = P.r.perm ? P.r.perm[i] : i;
+              if (iorig >= P.r.n) continue;  // a permutation entry out of range: skip the row
+              const bool ok =
+                  cvalid && pgood && (P.mode == MODE_CROSS || (P.mode == MODE_PDIST ? cj < i : cj <= i));
+              if (!__any_sync(FULL, ok)) continue;  // alike in every window
+              const uint64_t roff = P.r.off[iorig];
+              const uint32_t rpoints = (uint32_t)(P.r.off[iorig + 1] - roff), rlen = P.r.lens[iorig];
+              const uint64_t* rtime = P.r.times + roff;
+              const V* rval = rvals + roff;
+
+              A acc;
+              uint64_t* cslot = carry + (size_t)r * FIXED_CARRY * 32 + lane;
+              if (!first) acc.restore(cslot);
+              uint32_t k0 = rk0[r], z, m;
+              uint64_t Ap = Ab;
+              bool first_piece = true;
+              for (;;)
+              {
+                // up to X of the row's elements from k0: z of them end by Ap
+                // (skipped), c2 before Be
+                uint32_t avail, c2;
+                for (;;)
+                {
+                  avail = min(X, rlen - k0);
+                  uint32_t zl = 0, cl = 0;
+                  for (uint32_t k = lane; k < avail; k += 32)
+                  {
+                    const uint64_t e = rtime[k0 + k];
+                    rv[k] = rval[k0 + k];
+                    rt[k] = e;
+                    zl += e <= Ap ? 1u : 0u;
+                    cl += e < Be ? 1u : 0u;
+                  }
+                  z = __reduce_add_sync(FULL, zl);
+                  c2 = __reduce_add_sync(FULL, cl);
+                  if (z < avail) break;
+                  k0 += avail;  // all of them end by Ap; the last element of a row ends at END
+                  __syncwarp();
+                }
+                const bool full = c2 + 1 <= avail;  // the piece reaches Be
+                m = full ? (c2 + 1 > z ? c2 + 1 - z : 1u) : avail - z;
+                __syncwarp();
+                const uint64_t Bp = full ? Be : rt[avail - 1];
+                const V vlast = rv[z + m - 1];
+                __syncwarp();
+                if (lane <= U)  // z + m + U <= X + U < RB
+                {
+                  rv[z + m - 1 + lane] = vlast;
+                  rt[z + m - 1 + lane] = Bp;
+                }
+                __syncwarp();
+                // this lane's column elements meeting [Ap, Bp)
+                uint32_t g0 = 0, g1 = cm - 1;
+                if (!first_piece) g0 = column_find<true>(lcol, CS, 0, g1, Ap);
+                if (!full) g1 = column_find<false>(lcol, CS, g0, g1, Bp);
+                const uint32_t ncol = (first_piece && full) ? maxmc : __reduce_max_sync(FULL, g1 - g0 + 1);
+                walk(acc, rt + z, rv + z, (uint32_t)__cvta_generic_to_shared(lcol) + g0 * CS, vof, m, m + ncol - 1, Ap);
+                __syncwarp();
+                if (full) break;
+                k0 += z + m;
+                Ap = Bp;
+                first_piece = false;
+              }
+              if (lane == 0) rk0[r] = k0 + z + m - 1;  // the element reaching Be starts the next window
+              if (!last)
+              {
+                acc.save(cslot);
+                continue;
+              }
+
+              const double* rpts = P.r.pts + 2 * roff;
+              double res = acc.value() * unit;
+              // the last rectangle, to the largest double, where the PCFs'
+              // last values leave something of it
+              const double rlast = rpts[2 * rpoints - 1];
+              if (__any_sync(FULL, ((__double_as_longlong(rlast) | __double_as_longlong(clast)) << 1) != 0))
+              {
+                const double tail = op_f64<K>(rlast, clast);
+                if (tail != 0.0) res = fma(tail, tmax_of<double>(), res);
+              }
+              const uint64_t Tr = rlen > 1 ? rtime[rlen - 2] : 0, Tc = clen > 1 ? ctime[clen - 2] : 0;
+              const Shape rshape = P.r.shapes[iorig];
+              unsigned redo = __ballot_sync(FULL, ok && !acc.good(rshape, cshape, Tr > Tc ? Tr : Tc));
+              while (redo)
+              {
+                const int k = __ffs((int)redo) - 1;
+                redo &= redo - 1;
+                const uint64_t o = __shfl_sync(FULL, coff, k);
+                const double x = direct_pair<K>(rpts, rpoints, P.c.pts + 2 * o, __shfl_sync(FULL, cpoints, k));
+                if (lane == k) res = x;
+              }
+              if (ok)
+              {
+                if (K == OPK_L2DIST) res = sqrt(res);
+                const uint64_t idx = P.mode == MODE_CROSS ? iorig * P.ld + corig : condensed_index(P.mode, iorig, corig);
+                const uint64_t rel = idx - P.out_base;  // wraps for idx < out_base
+                if (rel < P.out_count) P.out[rel] = res;
+              }
+            }
+            __syncthreads();
+            if (last) break;
+            Ab = Be;
+            first = false;
+          }
+        }
+        __syncthreads();
+      }
+    }
+
+    template <int K>
+    __global__ void __launch_bounds__(FIXED_WARPS * 32, 1) fixed_pairs_kernel(const __grid_constant__ FixedParams P)
+    {
+      extern __shared__ __align__(16) unsigned char smem_raw[];
+      const Form f = form_of(*P.rec, K);
+      if (f.kind == 1)
+      {
+        if (K == OPK_INNER && f.sign) run_items<K, Counts<K, K == OPK_INNER>>(P, f, smem_raw);
+        else run_items<K, Counts<K, false>>(P, f, smem_raw);
+      }
+      else if (f.kind == 2)
+      {
+        if (K == OPK_INNER && f.sign) run_items<K, General<K, K == OPK_INNER>>(P, f, smem_raw);
+        else run_items<K, General<K, false>>(P, f, smem_raw);
+      }
+    }
+  }
+
+  // ---- launchers ----------------------------------------------------------------
+
+  cudaError_t launch_fixed_record(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap, FixedRecord* rec,
+                                  int sms, cudaStream_t st)
+  {
+    if (n == 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 8);
+    fixed_record_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, rec);
+    return launched();
+  }
+
+  cudaError_t launch_fixed_pack(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
+                                const FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
+                                bool elements, unsigned* gate, int sms, cudaStream_t st)
+  {
+    if (n == 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 8);
+    fixed_pack_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, rec, opk, packed, shapes, lens, elements, gate);
+    return launched();
+  }
+
+  cudaError_t launch_fixed_pairs(const FixedParams& P, int opk, int grid, cudaStream_t st)
+  {
+    void (*fn)(const FixedParams) = opk == OPK_L1       ? fixed_pairs_kernel<OPK_L1>
+                                    : opk == OPK_L2DIST ? fixed_pairs_kernel<OPK_L2DIST>
+                                    : opk == OPK_INNER  ? fixed_pairs_kernel<OPK_INNER>
+                                                        : nullptr;
+    if (!fn) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_bytes);
+    if (e != cudaSuccess) return e;
+    fn<<<grid, FIXED_WARPS * 32, P.smem_bytes, st>>>(P);
+    return launched();
+  }
+}

@@ -283,6 +283,8 @@ namespace sbg
     const int nwarps = blockDim.x >> 5;
     Elem<T>* rbuf = rows + (size_t)warp * L.row_cap;
     const T TM = tmax_of<T>();
+    if constexpr (sizeof(T) == 8)
+      if (L.gate && *L.gate) return;
 
     for (;;)
     {
@@ -864,6 +866,8 @@ namespace sbg
     const int warp = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
 
+    if constexpr (sizeof(T) == 8)
+      if (L.gate && *L.gate) return;
     for (;;)
     {
       if (threadIdx.x == 0)

@@ -225,10 +225,12 @@ namespace sbg
 
   // Length order (sort.cu): within each window of LENGTH_ORDER_WINDOW
   // consecutive PCFs, by breakpoint count, ties by index.  The device
-  // version; `scratch` holds length_order_scratch_bytes(n) bytes.
+  // version; `scratch` holds length_order_scratch_bytes(n) bytes.  With
+  // `lens`, by those lengths instead of the offsets' own.
   constexpr uint64_t LENGTH_ORDER_WINDOW = 1024;
   uint64_t length_order_scratch_bytes(uint64_t n);
-  void length_order_device(const uint64_t* off, uint64_t n, uint32_t* perm, void* scratch, cudaStream_t st);
+  void length_order_device(const uint64_t* off, uint64_t n, uint32_t* perm, void* scratch, cudaStream_t st,
+                           const uint32_t* lens = nullptr);
 
   // Launch accounting: every kernel launch of the library is followed by
   // launched(), which counts it and returns the launch error.  A CUDA graph

@@ -41,7 +41,9 @@ namespace sbg
     // needs the warp's own barrier after a stage of the same kind; a block
     // barrier precedes every stage that crosses warps and the stage after it.
     // The last window is padded with all-ones keys, which sort last.
-    __global__ void __launch_bounds__(SORT_THREADS) window_order_kernel(const uint64_t* __restrict__ off, uint64_t n,
+    // With `lens`, by those lengths instead of the offsets' own.
+    __global__ void __launch_bounds__(SORT_THREADS) window_order_kernel(const uint64_t* __restrict__ off,
+                                                                        const uint32_t* __restrict__ lens, uint64_t n,
                                                                         uint32_t* __restrict__ perm)
     {
       __shared__ uint64_t s[LENGTH_ORDER_WINDOW];
@@ -52,7 +54,7 @@ namespace sbg
         uint64_t key = ~0ull;
         if (g < n)
         {
-          uint64_t len = off[g + 1] - off[g];
+          uint64_t len = lens ? lens[g] : off[g + 1] - off[g];
           if (len > 0xffffffffull) len = 0xffffffffull;
           key = (len << 10) | i;
         }
@@ -81,12 +83,12 @@ namespace sbg
   // The order needs no global scratch; kept for callers that size one.
   uint64_t length_order_scratch_bytes(uint64_t) { return 0; }
 
-  void length_order_device(const uint64_t* off, uint64_t n, uint32_t* perm, void*, cudaStream_t st)
+  void length_order_device(const uint64_t* off, uint64_t n, uint32_t* perm, void*, cudaStream_t st, const uint32_t* lens)
   {
     if (n == 0) return;
     if (n > 0xffffffffull) throw Error(ST_INVALID_ARGUMENT, "too many PCFs for a 32-bit processing order");
     const uint64_t windows = (n + LENGTH_ORDER_WINDOW - 1) / LENGTH_ORDER_WINDOW;
-    window_order_kernel<<<(unsigned)windows, SORT_THREADS, 0, st>>>(off, n, perm);
+    window_order_kernel<<<(unsigned)windows, SORT_THREADS, 0, st>>>(off, lens, n, perm);
     SBG_CUDA(launched());
   }
 }
