@@ -252,7 +252,7 @@ namespace sbg
   static BatchBase* make_batch(int op, double p, int mode, const sbg_problem* probs, uint64_t n, int flags)
   {
     std::unique_ptr<Batch<T>> b(new Batch<T>);
-    b->op = op; b->p = p; b->mode = mode; b->opk = op_kind(op, p);
+    b->op = op; b->p = p; b->mode = mode; b->opk = settings().variant.load() == 0 ? power_kind(op_kind(op, p), p) : op_kind(op, p);
     b->use_graph = (flags & SBG_BATCH_GRAPH) != 0;
     b->tune_window = (flags & SBG_BATCH_TUNE_WINDOW) != 0;
     b->dev = device_info();

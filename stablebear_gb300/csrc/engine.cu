@@ -259,6 +259,9 @@ namespace sbg
     throw Error(ST_INVALID_ARGUMENT, "unknown op " + std::to_string(op));
   }
 
+  // The kernel an automatic call launches; a forced variant keeps pow().
+  static int launch_kind(int opk, double p) { return settings().variant.load() == 0 ? power_kind(opk, p) : opk; }
+
   uint64_t output_count(int mode, uint64_t nr, uint64_t nc)
   {
     if (mode == MODE_PDIST) return nr == 0 ? 0 : nr * (nr - 1) / 2;
@@ -890,7 +893,7 @@ namespace sbg
         d.ccap = ctot;
       }
     }
-    launch_problem<T>(d, pl, opk, st);
+    launch_problem<T>(d, pl, launch_kind(opk, p), st);
   }
 
   template void compute_device<float>(int, int, double, const PcfSet<float>&, const PcfSet<float>*, const uint32_t*,
@@ -966,7 +969,7 @@ namespace sbg
         d.ccap = col_points;
       }
     }
-    launch_problem<T>(d, pl, opk, st, reinterpret_cast<unsigned long long*>(base));
+    launch_problem<T>(d, pl, launch_kind(opk, p), st, reinterpret_cast<unsigned long long*>(base));
   }
 
   template size_t scratch_needed<float>(int, uint64_t, uint64_t, uint32_t, uint64_t, uint64_t);
@@ -1277,7 +1280,7 @@ namespace sbg
           return;
         }
       }
-      launch_problem<T>(d, pl, opk, bs);
+      launch_problem<T>(d, pl, launch_kind(opk, p), bs);
       SBG_CUDA(cudaEventRecord(computed[b].e, bs));
     };
 

@@ -988,9 +988,22 @@ namespace sbg
       case OPK_L1: fn = pairs_kernel<T, OPK_L1, U, VAR>; break;
       case OPK_L2DIST: fn = pairs_kernel<T, OPK_L2DIST, U, VAR>; break;
       case OPK_LP: fn = pairs_kernel<T, OPK_LP, U, VAR>; break;
+      case OPK_POW + 3:
+        if constexpr (VAR == 5) fn = pairs_kernel<T, OPK_POW + 3, U, VAR>;
+        break;
+      case OPK_POW + 5:
+        if constexpr (VAR == 5) fn = pairs_kernel<T, OPK_POW + 5, U, VAR>;
+        break;
+      case OPK_POW + 6:
+        if constexpr (VAR == 5) fn = pairs_kernel<T, OPK_POW + 6, U, VAR>;
+        break;
+      case OPK_POW + 8:
+        if constexpr (VAR == 5) fn = pairs_kernel<T, OPK_POW + 8, U, VAR>;
+        break;
       case OPK_INNER: fn = pairs_kernel<T, OPK_INNER, U, VAR>; break;
-      default: return cudaErrorInvalidValue;
+      default: break;
     }
+    if (!fn) return cudaErrorInvalidValue;
     if (VAR != 0)
     {
       cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1010,6 +1023,10 @@ namespace sbg
       case OPK_L1: fn = pairs_hybrid_kernel<T, OPK_L1, U>; break;
       case OPK_L2DIST: fn = pairs_hybrid_kernel<T, OPK_L2DIST, U>; break;
       case OPK_LP: fn = pairs_hybrid_kernel<T, OPK_LP, U>; break;
+      case OPK_POW + 3: fn = pairs_hybrid_kernel<T, OPK_POW + 3, U>; break;
+      case OPK_POW + 5: fn = pairs_hybrid_kernel<T, OPK_POW + 5, U>; break;
+      case OPK_POW + 6: fn = pairs_hybrid_kernel<T, OPK_POW + 6, U>; break;
+      case OPK_POW + 8: fn = pairs_hybrid_kernel<T, OPK_POW + 8, U>; break;
       case OPK_INNER: fn = pairs_hybrid_kernel<T, OPK_INNER, U>; break;
       default: return cudaErrorInvalidValue;
     }
@@ -1030,6 +1047,10 @@ namespace sbg
       case OPK_L1: fn = pairs_window_kernel<T, OPK_L1, U>; break;
       case OPK_L2DIST: fn = pairs_window_kernel<T, OPK_L2DIST, U>; break;
       case OPK_LP: fn = pairs_window_kernel<T, OPK_LP, U>; break;
+      case OPK_POW + 3: fn = pairs_window_kernel<T, OPK_POW + 3, U>; break;
+      case OPK_POW + 5: fn = pairs_window_kernel<T, OPK_POW + 5, U>; break;
+      case OPK_POW + 6: fn = pairs_window_kernel<T, OPK_POW + 6, U>; break;
+      case OPK_POW + 8: fn = pairs_window_kernel<T, OPK_POW + 8, U>; break;
       case OPK_INNER: fn = pairs_window_kernel<T, OPK_INNER, U>; break;
       default: return cudaErrorInvalidValue;
     }
