@@ -25,9 +25,11 @@
 // adds: the summation order is not deterministic.
 #include "../../include/sbgpu.h"
 #include "sbg_internal.hpp"
+#include "backward_l2.cuh"
 
 #include <algorithm>
 #include <memory>
+#include <type_traits>
 
 namespace sbg
 {
@@ -50,7 +52,15 @@ namespace sbg
     uint32_t row_cap;       // per-warp shared gradient buffer (elements)
     uint32_t cols_cap;      // staged column elements per lane (0: columns read through L1)
     const uint32_t* perm;   // processing order -> PCF index (the windowed length order), or null
+    const unsigned* gate;   // nothing to do unless one of these three device words is set; null: no gate
+    const float* norm;      // with a gate: the PCFs' norms, for the close pairs
   };
+
+  // Whether a gated kernel has nothing to do: the contraction of
+  // backward_l2.cu has the call; or only the pairs it leaves out, for which
+  // the third word stands.
+  __device__ __forceinline__ bool closed(const unsigned* gate) { return gate && !(gate[0] | gate[1] | gate[2]); }
+  __device__ __forceinline__ bool close_only(const unsigned* gate) { return gate && !(gate[0] | gate[1]); }
 
   namespace
   {
@@ -450,10 +460,18 @@ namespace sbg
   // elements per column), so the walk reads them with conflict-free shared
   // loads instead of one L1 request of 8 sectors per warp-step; the host
   // picks it when the columns and the slots of 32 warps fit.
-  template <typename T, int OP, int W, bool STAGED>
+  // GATED: behind the contraction (float32 L2 gradients); a kernel of its own,
+  // because the gate's tests cost the other calls up to 2 %.
+  template <typename T, int OP, int W, bool STAGED, bool GATED = false>
   __global__ void __launch_bounds__(STAGED ? 1024 : 512) pairs_backward_window_kernel(
       const __grid_constant__ BwdParams<T> B)
   {
+    bool only = false;  // the close pairs alone
+    if constexpr (GATED)
+    {
+      if (closed(B.gate)) return;
+      only = OP == BWD_L2DIST && close_only(B.gate);
+    }
     static_assert(W >= 1 && W <= 16, "two lanes per window element");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ unsigned long long s_item;
@@ -532,6 +550,8 @@ namespace sbg
             {
               const T D = B.fwd[idx];
               w = D > T(0) ? w / D : T(0);
+              if constexpr (GATED)
+                if (only && !l2_close((float)D, B.norm[iorig], B.norm[corig])) w = T(0);
             }
           }
           const bool live = w != T(0);
@@ -656,10 +676,12 @@ namespace sbg
   // (dL/dv_k, dL/dt_{k+1}) slots to the point layout (dL/dt_k, dL/dv_k).
   // The slot of a PCF's last element holds no time gradient (there is no
   // breakpoint after it).  One warp per PCF.
-  template <typename T>
+  template <typename T, bool GATED>
   __global__ void pair_to_point_layout(const T* __restrict__ gp, const uint64_t* __restrict__ off, uint64_t n,
-                                       uint64_t npts, T* __restrict__ grad)
+                                       uint64_t npts, T* __restrict__ grad, const unsigned* gate)
   {
+    if (GATED && closed(gate)) return;
+    const bool add = GATED && close_only(gate);  // to what the contraction gave
     const uint64_t wid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
@@ -669,8 +691,9 @@ namespace sbg
       if (o + len > npts) continue;
       for (uint64_t k = lane; k < len; k += 32)
       {
-        grad[2 * (o + k)] = k == 0 ? T(0) : gp[2 * (o + k - 1) + 1];
-        grad[2 * (o + k) + 1] = gp[2 * (o + k)];
+        const T dt = k == 0 ? T(0) : gp[2 * (o + k - 1) + 1], dv = gp[2 * (o + k)];
+        grad[2 * (o + k)] = add ? grad[2 * (o + k)] + dt : dt;
+        grad[2 * (o + k) + 1] = add ? grad[2 * (o + k) + 1] + dv : dv;
       }
     }
   }
@@ -679,8 +702,10 @@ namespace sbg
   // d/dt_k = v_{k-1}^2 - v_k^2, weighted by dL/dK_ii.  One warp per PCF.
   template <typename T>
   __global__ void diag_backward_kernel(const Elem<T>* __restrict__ pk, const uint64_t* __restrict__ off, uint64_t n,
-                                       uint64_t npts, const T* __restrict__ grad_out, T* __restrict__ grad)
+                                       uint64_t npts, const T* __restrict__ grad_out, T* __restrict__ grad,
+                                       const unsigned* gate)
   {
+    if (closed(gate)) return;
     const uint64_t wid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
@@ -702,6 +727,25 @@ namespace sbg
         }
       }
     }
+  }
+
+  template <typename T>
+  __global__ void clear_kernel(T* __restrict__ p, uint64_t count, const unsigned* gate)
+  {
+    if (closed(gate)) return;
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < count; k += (uint64_t)gridDim.x * blockDim.x)
+      p[k] = T(0);
+  }
+
+  // The walk that can run gated behind the contraction.
+  constexpr bool default_walk()
+  {
+#if defined(SBG_BWD_LEGACY) || defined(SBG_BWD_ROWSYNC) || defined(SBG_BWD_SQUARE) || \
+    defined(SBG_BWD_SQUARE_COLUMNS) || defined(SBG_BWD_WARP_ITEMS) || defined(SBG_BWD_STAGE_COLUMNS)
+    return false;
+#else
+    return true;
+#endif
   }
 
   constexpr bool defined_stage_columns()
@@ -742,8 +786,41 @@ namespace sbg
     // 32 columns of a group then have similar lengths, so the warp-uniform
     // step count wastes little.  Gradients land at the PCFs' own offsets.
     length_order_device(off, n, static_cast<uint32_t*>(order), nullptr, st);
-    SBG_CUDA(cudaMemsetAsync(paired, 0, std::max<uint64_t>(1, npts) * 2 * sizeof(T), st));
-    SBG_CUDA(launch_pack<T>(pts, off, n, static_cast<Elem<T>*>(packed), npts, dev.sms, st));
+
+    // Float L2 gradients as a contraction (backward_l2.cu); the walk below
+    // then runs behind it, gated: it does its work where the data or the
+    // weights did not suit.
+    const unsigned* gate = nullptr;
+    const float* norms = nullptr;
+    std::unique_ptr<StreamBuffer> l2;
+    if constexpr (sizeof(T) == 4 && default_walk())
+    {
+      if (bop != BWD_L1DIST)
+      {
+        const L2BackwardPlan plan = l2_backward_plan(n, npts, dev);
+        if (plan.ok)
+        {
+          try { l2.reset(new StreamBuffer(plan.bytes, st)); }
+          catch (const Error& e)
+          {
+            if (e.status != ST_OUT_OF_MEMORY) throw;  // the walk needs less
+          }
+          if (l2)
+            gate = l2_backward(plan, l2->get(), pts, off, n, npts, grad_out, bop == BWD_L2DIST ? fwd : nullptr,
+                               static_cast<const uint32_t*>(order), grad, &norms, dev, st);
+        }
+      }
+    }
+
+    if (gate)
+    {
+      const unsigned blocks = (unsigned)std::min<uint64_t>((npts * 2 + 1023) / 1024, (uint64_t)dev.sms * 4);
+      clear_kernel<T><<<std::max(1u, blocks), 256, 0, st>>>(static_cast<T*>(paired), npts * 2, gate);
+      SBG_CUDA(launched());
+    }
+    else
+      SBG_CUDA(cudaMemsetAsync(paired, 0, std::max<uint64_t>(1, npts) * 2 * sizeof(T), st));
+    SBG_CUDA(launch_pack<T>(pts, off, n, static_cast<Elem<T>*>(packed), npts, dev.sms, st, gate));
 
     BwdParams<T> B{};
     B.pk = static_cast<const Elem<T>*>(packed);
@@ -752,6 +829,8 @@ namespace sbg
     B.queue = static_cast<unsigned long long*>(queue);
     B.row_cap = lmax;
     B.perm = static_cast<const uint32_t*>(order);
+    B.gate = gate;
+    B.norm = norms;
     // As many warps (up to 32) as the per-warp row-gradient buffers allow:
     // the merge is latency-bound, so occupancy pays.  Columns are read
     // through L1: staging them in shared memory (behind
@@ -880,6 +959,20 @@ namespace sbg
                     : (bop == BWD_INNER ? pairs_backward_kernel<T, BWD_INNER, SIDE, WI>
                        : bop == BWD_L2DIST ? pairs_backward_kernel<T, BWD_L2DIST, SIDE, WI>
                                            : pairs_backward_kernel<T, BWD_L1DIST, SIDE, WI>);
+      if constexpr (sizeof(T) == 4 && default_walk())
+      {
+        if (gate)
+        {
+          auto gated = [&](auto op) {
+            constexpr int OP = decltype(op)::value;
+            fn = BWD_WS == 12  ? pairs_backward_window_kernel<T, OP, 12, true, true>
+                 : BWD_WS == 8 ? pairs_backward_window_kernel<T, OP, 8, true, true>
+                               : pairs_backward_window_kernel<T, OP, BWD_W, false, true>;
+          };
+          if (bop == BWD_INNER) gated(std::integral_constant<int, BWD_INNER>{});
+          else gated(std::integral_constant<int, BWD_L2DIST>{});
+        }
+      }
       SBG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       // persistent CTAs: as many per SM as registers, threads and shared memory allow
       int per_sm = 1;
@@ -891,14 +984,17 @@ namespace sbg
     }
     {
       const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)dev.sms * 8);
-      pair_to_point_layout<T><<<blocks, 256, 0, st>>>(static_cast<const T*>(paired), off, n, npts, grad);
+      if (gate)
+        pair_to_point_layout<T, true><<<blocks, 256, 0, st>>>(static_cast<const T*>(paired), off, n, npts, grad, gate);
+      else
+        pair_to_point_layout<T, false><<<blocks, 256, 0, st>>>(static_cast<const T*>(paired), off, n, npts, grad, gate);
       SBG_CUDA(launched());
     }
     if (bop == BWD_INNER)
     {
       // after the layout pass on the same stream: plain adds are race-free
       const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)dev.sms * 8);
-      diag_backward_kernel<T><<<blocks, 256, 0, st>>>(B.pk, off, n, npts, grad_out, grad);
+      diag_backward_kernel<T><<<blocks, 256, 0, st>>>(B.pk, off, n, npts, grad_out, grad, gate);
       SBG_CUDA(launched());
     }
   }

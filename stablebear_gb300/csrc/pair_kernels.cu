@@ -956,8 +956,9 @@ namespace sbg
   // CSR offset) holds (v_k, t_{k+1}), the last one (v_{L-1}, TMAX).
   template <typename T>
   __global__ void pack_segments_kernel(const T* __restrict__ pts, const uint64_t* __restrict__ off, uint64_t n,
-                                       Elem<T>* __restrict__ out, uint64_t cap)
+                                       Elem<T>* __restrict__ out, uint64_t cap, const unsigned* gate)
   {
+    if (gate && !(gate[0] | gate[1] | gate[2])) return;
     const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
@@ -1080,22 +1081,22 @@ namespace sbg
 
   template <typename T>
   cudaError_t launch_pack(const T* pts, const uint64_t* off, uint64_t n, Elem<T>* out, uint64_t cap, int sms,
-                          cudaStream_t s)
+                          cudaStream_t s, const unsigned* gate)
   {
     if (n == 0) return cudaSuccess;
     uint64_t blocks = (n + 7) / 8;
     const uint64_t max_blocks = (uint64_t)sms * 8;
     if (blocks > max_blocks) blocks = max_blocks;
-    pack_segments_kernel<T><<<(unsigned)blocks, 256, 0, s>>>(pts, off, n, out, cap);
+    pack_segments_kernel<T><<<(unsigned)blocks, 256, 0, s>>>(pts, off, n, out, cap, gate);
     return launched();
   }
 
   template cudaError_t launch_pairs<float>(const LaunchParams<float>&, int, int, int, int, size_t, cudaStream_t);
   template cudaError_t launch_pairs<double>(const LaunchParams<double>&, int, int, int, int, size_t, cudaStream_t);
   template cudaError_t launch_pack<float>(const float*, const uint64_t*, uint64_t, Elem<float>*, uint64_t, int,
-                                          cudaStream_t);
+                                          cudaStream_t, const unsigned*);
   template cudaError_t launch_pack<double>(const double*, const uint64_t*, uint64_t, Elem<double>*, uint64_t, int,
-                                           cudaStream_t);
+                                           cudaStream_t, const unsigned*);
 
   int kernel_unroll(bool f64) { return f64 ? Unroll<double>::value : Unroll<float>::value; }
 }

@@ -175,7 +175,7 @@ namespace sbg
                            size_t smem_bytes, cudaStream_t s);
   template <typename T>
   cudaError_t launch_pack(const T* pts, const uint64_t* off, uint64_t n, Elem<T>* out, uint64_t cap, int sms,
-                          cudaStream_t s);
+                          cudaStream_t s, const unsigned* gate = nullptr);  // gate: only where one of three words is set
   int kernel_unroll(bool f64);
 
   // Shared-memory layout of the time-windowed variant for `warps` warps and
