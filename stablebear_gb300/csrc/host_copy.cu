@@ -9,10 +9,12 @@
 #include "host_copy.hpp"
 
 #include <algorithm>
+#include <atomic>
 #include <condition_variable>
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <sys/mman.h>
 #include <thread>
 #include <unistd.h>
 #include <vector>
@@ -270,6 +272,51 @@ namespace sbg
     // the buffers are reused by the next upload: wait for the last DMAs
     SBG_CUDA(cudaEventSynchronize(p.ev[0]));
     SBG_CUDA(cudaEventSynchronize(p.ev[1]));
+  }
+
+  bool host_pages_mapped()
+  {
+    // per device; read once
+    static std::atomic<int> known[kUploadDevices] = {};
+    int dev = 0;
+    SBG_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kUploadDevices) return false;
+    int k = known[dev].load(std::memory_order_relaxed);
+    if (!k)
+    {
+      int pageable = 0, tables = 0;
+      host_memory_access(&pageable, &tables);
+      k = pageable && tables ? 2 : 1;
+      known[dev].store(k, std::memory_order_relaxed);
+    }
+    return k == 2;
+  }
+
+  bool make_pages(void* dst, size_t bytes)
+  {
+#ifdef MADV_POPULATE_WRITE
+    if (bytes == 0) return true;
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(dst) / page * page;
+    const uintptr_t hi = (reinterpret_cast<uintptr_t>(dst) + bytes + page - 1) / page * page;
+    auto make = [](uintptr_t a, uintptr_t b) {
+      return a >= b || madvise(reinterpret_cast<void*>(a), b - a, MADV_POPULATE_WRITE) == 0;
+    };
+    // Three threads are the most that gain (72 MB: 1.8 ms with one, 0.8 with
+    // three, 1.6 with sixteen; page by page with an atomic that keeps the
+    // byte, 21 ms); below 16 MB waking the pool costs what it saves.
+    constexpr unsigned THREADS = 3;
+    if (hi - lo < (16u << 20) || host_parts() < THREADS) return make(lo, hi);
+    const uintptr_t per = ((hi - lo) / THREADS / page + 1) * page;
+    std::atomic<bool> all{true};
+    host_parallel([&](unsigned k) {
+      if (k < THREADS && !make(lo + per * k, std::min(hi, lo + per * (k + 1)))) all = false;
+    });
+    return all;
+#else
+    (void)dst;
+    return bytes == 0;
+#endif
   }
 
   void host_memory_access(int* pageable, int* host_page_tables)

@@ -44,6 +44,14 @@ namespace sbg
   unsigned host_parts();
   void host_parallel(const std::function<void(unsigned)>& job);
 
+  // Whether the current device walks the host's page tables, so that copies
+  // to pageable memory run at the speed of pinned ones.
+  bool host_pages_mapped();
+
+  // Makes the pages of [dst, dst + bytes) exist and writable, contents kept;
+  // false where the kernel cannot.
+  bool make_pages(void* dst, size_t bytes);
+
   // cudaDevAttrPageableMemoryAccess / ...UsesHostPageTables of the current
   // device: 1/1 on coherent hosts (Grace + NVLink-C2C) where kernels may
   // store straight into malloc'd host memory.
