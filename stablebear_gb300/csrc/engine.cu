@@ -136,11 +136,12 @@ namespace sbg
   {
     reserve_bytes(bytes);
     void* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation)
+    cudaError_t e = cudaSuccess;
+    for (int attempt = 0; attempt < 2; ++attempt)
     {
-      pool_give_back();
       e = cudaMalloc(&p, bytes);
+      if (e != cudaErrorMemoryAllocation) break;
+      if (attempt == 0) pool_give_back();
     }
     if (e != cudaSuccess)
     {
