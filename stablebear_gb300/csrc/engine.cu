@@ -708,7 +708,19 @@ namespace sbg
     L.win_r = pl.win_r;
     L.row_slots = pl.row_slots;
     L.gate = gate;
-    const int grid = (int)std::min<uint64_t>((uint64_t)pl.grid, d.n_items);
+    // Few items (fewer than six per SM at 32 rows each): in length order a
+    // window's longest rows come last, and the longest items have to start
+    // first (N = 1000, L ~ U{10..200}: 88 us against 107).  With many, the
+    // last ones end the launch more evenly (N = 5000: 3.06 ms against 3.03).
+    // Up to 2.5 per SM, halves of 16 rows spread better than they cost in
+    // columns staged twice (N = 300: 38 us against 49, N = 800: 68 against
+    // 74; N = 1000, 3.5 per SM: 95 against 88; quarters are behind halves
+    // everywhere).  No pair's arithmetic depends on either.
+    const uint64_t sms = (uint64_t)device_info().sms;
+    L.last_first = pl.kvar == 5 && d.q == 1 && d.n_items < 6 * sms;
+    L.parts = L.last_first && 2 * d.n_items <= 5 * sms ? 2 : 1;
+    L.total_items = d.n_items * L.parts;
+    const int grid = (int)std::min<uint64_t>(std::max<uint64_t>(pl.grid, L.parts == 2 ? std::min<uint64_t>(L.total_items, sms * ctas_per_sm(device_info(), pl.warps, pl.smem_bytes)) : 1), L.total_items);
     SBG_CUDA(launch_pairs<T>(L, opk, pl.kvar, pl.warps, grid, pl.smem_bytes, st));
   }
 

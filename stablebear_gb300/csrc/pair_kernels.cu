@@ -301,12 +301,17 @@ namespace sbg
       const int mode = Pp->mode;
       const uint64_t nc = Pp->nc;
       const uint64_t G = ceil_div_u64(nc, 32);
-      const uint64_t local = item - Pp->item_begin;
+      const uint64_t local = L.last_first ? Pp->n_items - 1 - item / L.parts : item - Pp->item_begin;
       uint64_t c, g;
       if (mode == MODE_CROSS) { c = local / G; g = local % G; }
       else tri_decode(local, Pp->row_begin, Pp->row_end, Pp->q, G, &c, &g);
       uint64_t row_lo = Pp->row_begin + c * 32ull * Pp->q;
       uint64_t row_hi = row_lo + 32ull * Pp->q;
+      if (L.last_first)  // one of the parts of the chunk's 32 rows
+      {
+        row_lo += item % L.parts * (32 / L.parts);
+        row_hi = row_lo + 32 / L.parts;
+      }
       if (row_hi > Pp->row_end) row_hi = Pp->row_end;
       const uint64_t col0 = 32ull * g;
       if (mode != MODE_CROSS)

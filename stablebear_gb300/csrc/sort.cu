@@ -10,9 +10,8 @@
 // order is computed on the stream, with no host round trip.
 //
 // Keys (min(length, 2^32 - 1) << 10 | index in window) are unique within a
-// window, so a bitonic network (not stable by itself) gives the one
-// deterministic order.  Each window is keyed, sorted and written out by one
-// CTA in shared memory, in one launch.
+// window, so there is one order.  Windows are keyed, ranked and written out
+// in one launch.
 #include "../../include/sbgpu.h"
 #include "sbg_internal.hpp"
 
@@ -22,32 +21,26 @@ namespace sbg
 {
   namespace
   {
-    constexpr int SORT_THREADS = LENGTH_ORDER_WINDOW / 2;  // one compare-exchange per thread and stage
+    constexpr int SORT_THREADS = 256;
+    constexpr int SORT_PARTS = LENGTH_ORDER_WINDOW / 32;  // CTAs per window
 
-    __device__ __forceinline__ void cmp_swap(uint64_t& a, uint64_t& b, bool ascending)
-    {
-      if ((a > b) == ascending)
-      {
-        const uint64_t t = a;
-        a = b;
-        b = t;
-      }
-    }
-
-    // One CTA per window: keys (min(length, 2^32 - 1) << 10 | index in
-    // window) built from the offsets, a bitonic network in shared memory,
-    // the permutation written out.  A stage whose partner distance j is at
-    // most 32 pairs elements inside the 64 that one warp handles, so it only
-    // needs the warp's own barrier after a stage of the same kind; a block
-    // barrier precedes every stage that crosses warps and the stage after it.
-    // The last window is padded with all-ones keys, which sort last.
+    // Keys (min(length, 2^32 - 1) << 10 | index in window) of a whole window
+    // in shared memory; the place of a key is the number of keys below it.
+    // Each CTA places 32 of them, lane l of every warp counting for the l-th
+    // in that warp's eighth of the window.  (A bitonic network by one CTA per
+    // window is 55 dependent stages, 8.2 us against 5.1 at N = 1000.)
     // With `lens`, by those lengths instead of the offsets' own.
     __global__ void __launch_bounds__(SORT_THREADS) window_order_kernel(const uint64_t* __restrict__ off,
                                                                         const uint32_t* __restrict__ lens, uint64_t n,
                                                                         uint32_t* __restrict__ perm)
     {
-      __shared__ uint64_t s[LENGTH_ORDER_WINDOW];
-      const uint64_t base = (uint64_t)blockIdx.x * LENGTH_ORDER_WINDOW;
+      constexpr uint32_t EIGHTH = LENGTH_ORDER_WINDOW / (SORT_THREADS / 32);
+      __shared__ __align__(16) uint64_t s[LENGTH_ORDER_WINDOW];
+      __shared__ uint32_t place[32];
+      const uint64_t base = (uint64_t)(blockIdx.x / SORT_PARTS) * LENGTH_ORDER_WINDOW;
+      const uint32_t mine = (blockIdx.x % SORT_PARTS) * 32 + (threadIdx.x & 31);
+      if (base + (mine & ~31u) >= n) return;  // alike in the whole CTA
+      if (threadIdx.x < 32) place[threadIdx.x] = 0;
       for (uint32_t i = threadIdx.x; i < LENGTH_ORDER_WINDOW; i += SORT_THREADS)
       {
         const uint64_t g = base + i;
@@ -60,21 +53,19 @@ namespace sbg
         }
         s[i] = key;
       }
-      uint32_t prev_j = LENGTH_ORDER_WINDOW;  // the loads cross warps
-      for (uint32_t k = 2; k <= LENGTH_ORDER_WINDOW; k <<= 1)
-      {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1)
-        {
-          if (j >= 64 || prev_j >= 64) __syncthreads(); else __syncwarp();
-          const uint32_t t = threadIdx.x;
-          const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1));  // j is a power of two
-          cmp_swap(s[i], s[i + j], (i & k) == 0);
-          prev_j = j;
-        }
-      }
       __syncthreads();
-      for (uint32_t i = threadIdx.x; i < LENGTH_ORDER_WINDOW; i += SORT_THREADS)
-        if (base + i < n) perm[base + i] = (uint32_t)(base + (s[i] & 1023));
+      const uint64_t key = s[mine];
+      const uint32_t k0 = threadIdx.x / 32 * EIGHTH;
+      uint32_t below = 0;
+#pragma unroll 8
+      for (uint32_t k = k0; k < k0 + EIGHTH; k += 2)
+      {
+        const ulonglong2 two = *reinterpret_cast<const ulonglong2*>(s + k);
+        below += (two.x < key ? 1u : 0u) + (two.y < key ? 1u : 0u);
+      }
+      atomicAdd(&place[threadIdx.x & 31], below);
+      __syncthreads();
+      if (threadIdx.x < 32 && base + mine < n) perm[base + place[threadIdx.x]] = (uint32_t)(base + mine);
     }
   }
 
@@ -88,7 +79,7 @@ namespace sbg
     if (n == 0) return;
     if (n > 0xffffffffull) throw Error(ST_INVALID_ARGUMENT, "too many PCFs for a 32-bit processing order");
     const uint64_t windows = (n + LENGTH_ORDER_WINDOW - 1) / LENGTH_ORDER_WINDOW;
-    window_order_kernel<<<(unsigned)windows, SORT_THREADS, 0, st>>>(off, lens, n, perm);
+    window_order_kernel<<<(unsigned)(windows * SORT_PARTS), SORT_THREADS, 0, st>>>(off, lens, n, perm);
     SBG_CUDA(launched());
   }
 }
