@@ -351,11 +351,13 @@ namespace sbg
     {
       pl.packed = false;
       pl.kvar = 6;
-      pl.warps = want_w > 0 ? std::min(want_w, 32) : 24;
+      pl.warps = want_w > 0 ? std::min(want_w, 32) : 32;
       // One cap for every shape the autotune tries (up to 32 warps and 4x
       // the rows per item), else the one that fits the starting shape.
       uint64_t qb = 1;
       for (uint64_t x : b->q_base) qb = std::max(qb, x);
+      if (!window_cap_allowed(es, pl.warps, (uint32_t)(32 * qb), b->usable))
+        throw Error(ST_INVALID_ARGUMENT, "batch: the window setting does not fit in shared memory");
       Plan probe;
       if (window_layout(probe, es, 32, (uint32_t)(32 * qb * 4), lmax, b->usable))
         b->win_cap = probe.lmax_c;
@@ -376,6 +378,15 @@ namespace sbg
     b->d_queue.reset(256);
     SBG_CUDA(cudaDeviceSynchronize());
     bool fit = false;
+    // The starting shape (autotune tries others; none changes a bit of a
+    // windowed result): 32 warps, and four times the rows per item where that
+    // leaves two items per SM, or one for short PCFs, whose items are mostly
+    // column staging.  24 problems, L ~ U{8..1024}: 8.18 ms with 128 rows,
+    // 8.33 with 32, 8.59 with 32 and 24 warps; 100 problems 37.3, 38.6, 39.8;
+    // 10 problems, L ~ U{8..200}: 0.93, 1.01, 1.04; 40 problems of up to 300
+    // PCFs, L ~ U{8..60}: 59 us, 85, 83.
+    if (b->windowed && want_w == 0)
+      fit = b->rebuild_items(32, 4) && b->total_items >= (uint64_t)b->dev.sms * (lmax <= 128 ? 1 : 2);
     for (int w = pl.warps; w >= 4 && !fit; w -= 4) fit = b->rebuild_items((uint32_t)w, 1);
     if (!fit) throw Error(ST_INVALID_ARGUMENT, "batch: the window setting does not fit in shared memory");
     return b.release();

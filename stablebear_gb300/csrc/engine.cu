@@ -504,7 +504,12 @@ namespace sbg
       pl.smem = true;
       pl.packed = false;
       pl.kvar = 6;
-      pl.warps = want_w > 0 ? std::min(want_w, 32) : 24;
+      // 32 warps, with windows of up to 440 elements beside their row
+      // buffers: N = 1021, L ~ U{16..512} 207 us, N = 4096 2.45 ms, N = 3000,
+      // L ~ U{8..1024} 2.61 ms; with 24 warps and row buffers padded for the
+      // longest column slice, which leave 344 elements: 237 us, 2.61 ms, 2.85
+      // ms; 32 warps and such buffers (280 elements): 213 us, 2.61, 2.79 ms.
+      pl.warps = want_w > 0 ? std::min(want_w, 32) : 32;
     }
 
     // Rows per item = 32 q: as large as possible (fewer column reloads,
@@ -539,7 +544,8 @@ namespace sbg
     if (pl.kvar == 6)
     {
       bool fit = false;
-      for (int w = pl.warps; w >= 4 && !fit; w -= 4)
+      const bool cap_ok = window_cap_allowed(es, pl.warps, 32 * q, usable);
+      for (int w = pl.warps; w >= 4 && !fit && cap_ok; w -= 4)
         fit = window_layout(pl, es, w, 32 * q, std::max(lmax_r, lmax_c), usable);
       if (!fit) throw Error(ST_INVALID_ARGUMENT, "time-windowed variant: the window setting does not fit in shared memory");
     }
@@ -579,12 +585,22 @@ namespace sbg
     return pl;
   }
 
+  bool window_cap_allowed(size_t es, int warps, uint32_t rows_per_item, size_t usable)
+  {
+    const size_t X = (size_t)std::max(0, settings().windowCap.load());
+    if (X == 0) return true;
+    if (warps < 4) return false;
+    const size_t slots = ((size_t)rows_per_item * 4 + 15) / 16 * 16;
+    const size_t row = 2 * X + (size_t)kernel_unroll(es == 16) + 1;
+    return 32 * X * es + (size_t)(4 + warps % 4) * row * es + slots <= usable;
+  }
+
   bool window_layout(Plan& pl, size_t es, int warps, uint32_t rows_per_item, uint32_t lmax, size_t usable,
                      uint32_t cap)
   {
     const uint32_t U = (uint32_t)kernel_unroll(es == 16);
     const size_t slots = ((size_t)rows_per_item * 4 + 15) / 16 * 16;
-    auto bytes = [&](uint32_t X) { return (size_t)32 * X * es + (size_t)warps * (2 * X + U + 1) * es + slots; };
+    auto bytes = [&](uint32_t X) { return (size_t)32 * X * es + (size_t)warps * (X + U + 1) * es + slots; };
     const uint32_t top = std::max<uint32_t>(8, (lmax + 7) / 8 * 8);
     uint32_t X = cap ? cap : (uint32_t)std::max(0, settings().windowCap.load());
     if (X == 0)
@@ -598,7 +614,7 @@ namespace sbg
     pl.warps = warps;
     pl.lmax_c = X;
     pl.win_r = X;
-    pl.row_cap = 2 * X + U + 1;
+    pl.row_cap = X + U + 1;
     pl.row_slots = rows_per_item;
     pl.smem_bytes = bytes(X);
     return true;
@@ -712,15 +728,21 @@ namespace sbg
     // window's longest rows come last, and the longest items have to start
     // first (N = 1000, L ~ U{10..200}: 88 us against 107).  With many, the
     // last ones end the launch more evenly (N = 5000: 3.06 ms against 3.03).
-    // Up to 2.5 per SM, halves of 16 rows spread better than they cost in
-    // columns staged twice (N = 300: 38 us against 49, N = 800: 68 against
-    // 74; N = 1000, 3.5 per SM: 95 against 88; quarters are behind halves
-    // everywhere).  No pair's arithmetic depends on either.
+    // Where the SMs would run dry, halves of 16 rows spread better than they
+    // cost in columns staged twice: up to 2.5 items per SM with two CTAs on
+    // each (N = 300: 38 us against 49, N = 800: 68 against 74; N = 1000, 3.5
+    // per SM: 95 against 88; quarters are behind halves everywhere), up to
+    // 0.75 with one, whose 32 warps have a row each already (L ~ U{16..512}:
+    // N = 300 77 us against 105, N = 600, 1.25 per SM, 121 against 107).  No
+    // pair's arithmetic depends on either.
     const uint64_t sms = (uint64_t)device_info().sms;
-    L.last_first = pl.kvar == 5 && d.q == 1 && d.n_items < 6 * sms;
-    L.parts = L.last_first && 2 * d.n_items <= 5 * sms ? 2 : 1;
+    const uint64_t resident = (uint64_t)ctas_per_sm(device_info(), pl.warps, pl.smem_bytes);
+    L.last_first = (pl.kvar == 5 || pl.kvar == 6) && d.q == 1 && d.n_items < 6 * sms;
+    L.parts = L.last_first && 4 * d.n_items <= (resident > 1 ? 10 : 3) * sms ? 2 : 1;
     L.total_items = d.n_items * L.parts;
-    const int grid = (int)std::min<uint64_t>(std::max<uint64_t>(pl.grid, L.parts == 2 ? std::min<uint64_t>(L.total_items, sms * ctas_per_sm(device_info(), pl.warps, pl.smem_bytes)) : 1), L.total_items);
+    uint64_t ctas = (uint64_t)pl.grid;  // what is resident, at most one per item
+    if (L.parts > 1) ctas = std::max<uint64_t>(ctas, sms * resident);
+    const int grid = (int)std::min<uint64_t>(ctas, L.total_items);
     SBG_CUDA(launch_pairs<T>(L, opk, pl.kvar, pl.warps, grid, pl.smem_bytes, st));
   }
 

@@ -470,7 +470,7 @@ namespace sbg
   // no side ever steps past its slice.  Integrals over [0, inf) split into
   // the window integrals exactly (the rectangles meeting a window are those
   // of the whole merge, cut at its ends).  Sums carry from piece to piece in
-  // registers and from window to window through the output element (raw
+  // registers, with their compensation, and from window to window through the output element (raw
   // sums, the finalizer after the last window), which the same CTA reads
   // back after a block barrier.
 
@@ -524,21 +524,24 @@ namespace sbg
     return moved;
   }
 
-  // merge_smem_soa over one window: starts at t0 with the running sum acc0,
-  // clips every rectangle to end at tend, returns the raw compensated sum.
+  // merge_smem_soa over one window or one piece of it: starts at t0, clips
+  // every rectangle to end at tend, continues the sum acc and its
+  // compensation.  m: the elements of the row's slice.
   template <typename T, int K, int U>
-  __device__ __forceinline__ T merge_window(const T* ft0, uint32_t voff, const Elem<T>* pg, uint32_t steps, T t0,
-                                            T tend, T acc0, T p)
+  __device__ __forceinline__ void merge_window(const T* ft0, uint32_t voff, const Elem<T>* pg, uint32_t m,
+                                               uint32_t steps, T t0, T tend, T& acc, T& comp, T p)
   {
     T fv = *reinterpret_cast<const T*>(reinterpret_cast<const unsigned char*>(ft0) + voff);
     T ft = *ft0;
     Elem<T> G = *pg;
     uint32_t af = (uint32_t)__cvta_generic_to_shared(ft0);
+    const uint32_t af_last = af + (m - 1) * (uint32_t)sizeof(T);
     uint32_t ag = (uint32_t)__cvta_generic_to_shared(pg);
-    T t = t0, acc = acc0, comp = T(0);
+    T t = t0;
     const uint32_t nblk = (steps + U - 1) / U;
     for (uint32_t b = 0; b < nblk; ++b)
     {
+      af = min(af, af_last);
       T blk = T(0);
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -550,7 +553,6 @@ namespace sbg
       }
       kahan_add(acc, comp, blk);
     }
-    return acc - comp;
   }
 
   // First k in [lo, hi] whose element of this lane's staged column ends
@@ -569,7 +571,12 @@ namespace sbg
   }
 
   // Shared memory: the column block (lmax_c x 32 elements, interleaved), one
-  // row buffer per warp (row_cap elements' bytes: times, then values), and the
+  // row buffer per warp (row_cap elements' bytes: times, then values, a slice
+  // and U sentinels: the row address is pulled back at each block start, as in
+  // the plain variant; a sentinel per step of the longest column slice halved
+  // the room and was as much to write as the slice: 24 problems, L ~
+  // U{8..1024}, 8.18 ms against 8.52, N = 10,000, L ~ U{16..489} 12.1 ms
+  // against 12.9), and the
   // saved slice start of each row of the item (row_slots words).
   template <typename T, int K, int U>
   __global__ void __launch_bounds__(1024, 1) pairs_window_kernel(const __grid_constant__ LaunchParams<T> L)
@@ -605,12 +612,17 @@ namespace sbg
       const int mode = Pp->mode;
       const uint64_t nc = Pp->nc;
       const uint64_t G = ceil_div_u64(nc, 32);
-      const uint64_t local = item - Pp->item_begin;
+      const uint64_t local = L.last_first ? Pp->n_items - 1 - item / L.parts : item - Pp->item_begin;
       uint64_t c, g;
       if (mode == MODE_CROSS) { c = local / G; g = local % G; }
       else tri_decode(local, Pp->row_begin, Pp->row_end, Pp->q, G, &c, &g);
       uint64_t row_lo = Pp->row_begin + c * 32ull * Pp->q;
       uint64_t row_hi = row_lo + 32ull * Pp->q;
+      if (L.last_first)  // one of the parts of the chunk's 32 rows
+      {
+        row_lo += item % L.parts * (32 / L.parts);
+        row_hi = row_lo + 32 / L.parts;
+      }
       if (row_hi > Pp->row_end) row_hi = Pp->row_end;
       const uint64_t col0 = 32ull * g;
       if (mode != MODE_CROSS)
@@ -715,7 +727,7 @@ namespace sbg
             else idx = condensed_index(mode, iorig, corig);
             const uint64_t rel = idx - Pp->out_base;  // wraps for idx < out_base
             const bool store = ok && rel < Pp->out_count;
-            T acc = (!first && store) ? Pp->out[rel] : T(0);
+            T acc = (!first && store) ? Pp->out[rel] : T(0), comp = T(0);
 
             // The row's elements meeting [A, B), at most RW at a time: a row
             // denser than the item's columns takes several pieces, each a
@@ -753,7 +765,7 @@ namespace sbg
               const T Bp = full ? B : rt[avail - 1];
               const T vlast = rv[z + m - 1];
               __syncwarp();
-              const uint32_t pad_end = z + m + maxmc + U;  // <= RW + CW + U < row_cap
+              const uint32_t pad_end = z + m + U;  // <= RW + U < row_cap
               for (uint32_t k = z + m - 1 + lane; k < pad_end; k += 32)
               {
                 rv[k] = vlast;
@@ -768,7 +780,8 @@ namespace sbg
               if (!first_piece) g0 = column_search<T, true>(cols, lane, 0, g1, Ap);
               if (!full) g1 = column_search<T, false>(cols, lane, g0, g1, Bp);
               const uint32_t ncol = (first_piece && full) ? maxmc : warp_max_u32(g1 - g0 + 1);
-              acc = merge_window<T, K, U>(rt + z, voff, cols + (size_t)g0 * 32 + lane, m + ncol - 1, Ap, Bp, acc, p);
+              merge_window<T, K, U>(rt + z, voff, cols + (size_t)g0 * 32 + lane, m, m + ncol - 1, Ap, Bp, acc, comp,
+                                    p);
               __syncwarp();
               if (full) break;
               k0 += z + m;
@@ -778,7 +791,7 @@ namespace sbg
             // the element reaching B starts the next window (skipped there if
             // it ends at B)
             if (lane == 0) rk0[r] = k0 + z + m - 1;
-            if (store) Pp->out[rel] = last ? PairOp<K>::fin(acc, p) : acc;
+            if (store) Pp->out[rel] = last ? PairOp<K>::fin(acc - comp, p) : acc - comp;
           }
           __syncthreads();
           if (last) break;

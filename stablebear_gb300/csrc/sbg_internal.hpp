@@ -185,6 +185,11 @@ namespace sbg
   bool window_layout(Plan& pl, size_t elem_bytes, int warps, uint32_t rows_per_item, uint32_t lmax, size_t usable,
                      uint32_t cap = 0);
 
+  // Whether a window cap set by the caller (none: yes) is one the engine
+  // takes: it has to leave room for row buffers of twice its elements at the
+  // fewest warps the layout is tried with (4 and the remainder of `warps`).
+  bool window_cap_allowed(size_t elem_bytes, int warps, uint32_t rows_per_item, size_t usable);
+
   // Control block of one host-side run (progress, cancellation).
   struct RunControl
   {
