@@ -512,31 +512,49 @@ namespace sbg
       pl.warps = want_w > 0 ? std::min(want_w, 32) : 32;
     }
 
-    // Rows per item = 32 q: as large as possible (fewer column reloads,
-    // less end-of-item idling) while keeping >= 6 items per SM.  At most
-    // 1024 rows, one processing-order window, so that bands of whole
-    // windows start on item boundaries.
+    // Two CTAs of 16 warps per SM, where their shared memory fits, overlap one
+    // CTA's column staging and row fills with the other's merges: small
+    // problems, up to 256 rows per item, take them (below).
+    const bool two_ctas = settings().warps.load() == 0 && settings().rowChunk.load() == 0 && pl.kvar == 5 &&
+                          pl.warps > 16 && ctas_per_sm(dev, 16, smem_for(16)) >= 2;
+    // Rows per item = 32 q: as large as possible (fewer column reloads) while
+    // enough items per SM are left to end evenly.  At most 1024 rows, one
+    // processing-order window, so that bands of whole windows start on item
+    // boundaries.  Six items per SM are enough for two CTAs on each; with one,
+    // small q gain more from their next doubling than uneven ends cost (plain,
+    // L ~ U{10..200} held to one CTA: N = 1500 177 us at q = 2, 3.9 items per
+    // SM, 230 at 1; N = 2500 397 at q = 4, 5.5 items, 466 at 2; windowed, L ~
+    // U{16..512}: N = 1500 373 us at q = 2, 3.9 items, 460 at 1; N = 2400 906
+    // at q = 4, 5.0 items, 940 at 2), and the long items of the windowed
+    // variant want more of them at large q (N = 6000 4.64 ms at q = 8, 4.75 at
+    // 16, 7.9 items; N = 7500 7.19 at 16, 7.64 at 32, 6.5 items; L ~
+    // Poisson(512): N = 9000 20.6 at 16, 20.9 at 32, 9.2 items, N = 20,000
+    // 99.6 at 16, 98.3 at 32, 43 items).  In tenths of an item:
     // The hybrid kernel reads rows through L1 and restages only its 32
     // columns per item, so big items buy it little but a ragged tail on
     // uneven lengths: at most 64 rows (f64 stable-rank N = 20,000, L2 kernel
     // / pdist: 1921 / 2458 ms against 2048 / 2533 ms with 1024 rows).
     const uint32_t q_top = pl.kvar == 3 ? 2u : 32u;
+    auto tenths = [&](uint32_t cand) -> uint64_t {
+      if (pl.kvar == 6) return cand == 2 ? 35 : cand == 4 ? 50 : cand == 16 ? 100 : cand == 32 ? 200 : 60;
+      if (pl.kvar == 5 && !two_ctas) return cand == 2 ? 20 : cand == 4 ? 30 : cand == 8 ? 40 : 60;
+      return 60;
+    };
     uint32_t q = (uint32_t)std::max(0, settings().rowChunk.load());
     if (q == 0)
     {
       q = 1;
       for (uint32_t cand = q_top; cand >= 1; cand /= 2)
       {
-        if (items_for(mode, 0, nr, nc, cand) >= (uint64_t)dev.sms * 6) { q = cand; break; }
+        if (10 * items_for(mode, 0, nr, nc, cand) >= (uint64_t)dev.sms * tenths(cand)) { q = cand; break; }
       }
     }
     pl.q = q;
-    // Problems too small for 6 items per SM even at 32 rows per item: two
-    // CTAs of 16 warps per SM, so one CTA's column staging and row fills
-    // overlap the other's merges (N = 1000: 123.5 against 141 us).
-    if (settings().warps.load() == 0 && settings().rowChunk.load() == 0 && pl.kvar == 5 && q == 1 &&
-        pl.warps > 16 && items_for(mode, 0, nr, nc, 1) < (uint64_t)dev.sms * 6 &&
-        ctas_per_sm(dev, 16, smem_for(16)) >= 2)
+    // L ~ U{10..200}: N = 1000 88 us against 112 with one CTA of 32 warps, N =
+    // 1500 162 against 218, N = 2500 376 against 450, N = 4000 892 against
+    // 911; with more rows per item there is no difference to rely on (N =
+    // 3000, 30,000 and 60,000 2-4 % faster, N = 10,000 2 % slower).
+    if (two_ctas && q <= 8)
     {
       pl.warps = 16;
       pl.smem_bytes = smem_for(16);
@@ -724,10 +742,15 @@ namespace sbg
     L.win_r = pl.win_r;
     L.row_slots = pl.row_slots;
     L.gate = gate;
-    // Few items (fewer than six per SM at 32 rows each): in length order a
-    // window's longest rows come last, and the longest items have to start
-    // first (N = 1000, L ~ U{10..200}: 88 us against 107).  With many, the
-    // last ones end the launch more evenly (N = 5000: 3.06 ms against 3.03).
+    // Few items (fewer than twelve per SM): in length order a window's longest
+    // rows come last, and the longest items have to start first (L ~
+    // U{10..200}: N = 1000 88 us against 107, N = 1500 162 against 181, N =
+    // 2000 253 against 277; windowed, L ~ U{16..512}: N = 1500 373 against
+    // 431, N = 4096 2376 against 2450).  With many items, or large ones in the
+    // plain variant (where they hide what is staged next, and the last chunk's
+    // diagonal items are the small ones), the last items end the launch more
+    // evenly (N = 3200, q = 4, two CTAs: 592 against 607; N = 4000, q = 8: 891
+    // against 928; N = 5000, q = 1: 3.03 ms against 3.06).
     // Where the SMs would run dry, halves of 16 rows spread better than they
     // cost in columns staged twice: up to 2.5 items per SM with two CTAs on
     // each (N = 300: 38 us against 49, N = 800: 68 against 74; N = 1000, 3.5
@@ -737,8 +760,8 @@ namespace sbg
     // pair's arithmetic depends on either.
     const uint64_t sms = (uint64_t)device_info().sms;
     const uint64_t resident = (uint64_t)ctas_per_sm(device_info(), pl.warps, pl.smem_bytes);
-    L.last_first = (pl.kvar == 5 || pl.kvar == 6) && d.q == 1 && d.n_items < 6 * sms;
-    L.parts = L.last_first && 4 * d.n_items <= (resident > 1 ? 10 : 3) * sms ? 2 : 1;
+    L.last_first = d.n_items < 12 * sms && (pl.kvar == 6 || (pl.kvar == 5 && d.q <= (resident > 1 ? 2 : 4)));
+    L.parts = L.last_first && d.q == 1 && 4 * d.n_items <= (resident > 1 ? 10 : 3) * sms ? 2 : 1;
     L.total_items = d.n_items * L.parts;
     uint64_t ctas = (uint64_t)pl.grid;  // what is resident, at most one per item
     if (L.parts > 1) ctas = std::max<uint64_t>(ctas, sms * resident);

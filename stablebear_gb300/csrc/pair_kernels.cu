@@ -307,7 +307,7 @@ namespace sbg
       else tri_decode(local, Pp->row_begin, Pp->row_end, Pp->q, G, &c, &g);
       uint64_t row_lo = Pp->row_begin + c * 32ull * Pp->q;
       uint64_t row_hi = row_lo + 32ull * Pp->q;
-      if (L.last_first)  // one of the parts of the chunk's 32 rows
+      if (L.parts > 1)  // one of the parts of the chunk's 32 rows
       {
         row_lo += item % L.parts * (32 / L.parts);
         row_hi = row_lo + 32 / L.parts;
@@ -618,7 +618,7 @@ namespace sbg
       else tri_decode(local, Pp->row_begin, Pp->row_end, Pp->q, G, &c, &g);
       uint64_t row_lo = Pp->row_begin + c * 32ull * Pp->q;
       uint64_t row_hi = row_lo + 32ull * Pp->q;
-      if (L.last_first)  // one of the parts of the chunk's 32 rows
+      if (L.parts > 1)  // one of the parts of the chunk's 32 rows
       {
         row_lo += item % L.parts * (32 / L.parts);
         row_hi = row_lo + 32 / L.parts;

@@ -227,8 +227,8 @@ namespace sbg
     uint32_t row_cap;            // per-warp row buffer capacity (elements)
     uint32_t win_r;              // time-windowed variant: elements of a row slice
     uint32_t row_slots;          // time-windowed variant: rows of an item with saved slice starts
-    bool last_first;             // plain and windowed variants, one problem of 32-row chunks: items from the last one down,
-    uint32_t parts;              // each cut into this many by rows
+    bool last_first;             // plain and windowed variants, one problem: items from the last one down,
+    uint32_t parts;              // each (of 32 rows, if more than 1) cut into this many by rows
     const unsigned* gate;        // double, plain and hybrid variants: nothing to do where this device word is
                                  // set (the fixed-point kernel has the call); NULL: no gate
   };

@@ -11,7 +11,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [2, 16, 17, 33, 48, 300, 860, 900, 1340, 1380])
+@pytest.mark.parametrize("n", [2, 16, 17, 33, 48, 300, 860, 900, 1340, 1380, 2000, 2900])
 def test_parts_and_reversed_items_change_no_bit(n):
     import stablebear_gb300 as sb
     from stablebear_gb300 import synthetic
@@ -24,7 +24,7 @@ def test_parts_and_reversed_items_change_no_bit(n):
 
     got = run()
     try:
-        sb.set_tuning(row_chunk=2)
+        sb.set_tuning(row_chunk=8)
         want = run()
         sb.set_tuning(order=1)
         caller = run()
@@ -37,7 +37,7 @@ def test_parts_and_reversed_items_change_no_bit(n):
 
 # Longer PCFs take the windowed kernel, whose windows follow from the column
 # group: the same groups, so the same order, on both sides.
-@pytest.mark.parametrize("n", [2, 16, 17, 33, 48, 300, 430, 480, 1340, 1380])
+@pytest.mark.parametrize("n", [2, 16, 17, 33, 48, 300, 430, 480, 1340, 1380, 2100])
 def test_windowed_parts_and_reversed_items_change_no_bit(n):
     import stablebear_gb300 as sb
     from stablebear_gb300 import synthetic
@@ -50,7 +50,7 @@ def test_windowed_parts_and_reversed_items_change_no_bit(n):
 
     got = run()
     try:
-        sb.set_tuning(row_chunk=2)
+        sb.set_tuning(row_chunk=8)
         want = run()
     finally:
         sb.set_tuning()
