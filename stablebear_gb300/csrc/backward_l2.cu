@@ -19,7 +19,7 @@
 // Work per PCF pair falls from the merge's 2 L steps, with an atomic each, to
 // 2 bins FMAs and L^2 / bins list entries.  Nothing is added atomically, and
 // the sums are shorter.  N = 4096, L ~ U{16..512}, L2 kernel, forward and
-// backward: 14.4 -> 5.0 ms (the forward is 2.6 of it), error of the gradient
+// backward: 14.4 -> 4.8 ms (the forward is 2.4 of it), error of the gradient
 // 8.5e-7 -> 3.1e-7.
 //
 // For distances each bin's mean value over the PCFs is taken off first: only
