@@ -26,7 +26,7 @@ namespace sbg
 
   // A PCF's integer values (general form: over 2^32): sum of |changes|, of
   // their squares, and the largest |value|.
-  struct alignas(16) Shape { float tv, qv, vmax, pad; };
+  struct alignas(16) Shape { float tv, qv, vmax, close; };
 
   // One side's PCFs: CSR, processing order, and the packed arrays of `cap`
   // elements (times, then values).

@@ -106,6 +106,35 @@ def test_exact_sums_do_not_depend_on_order_bands_or_sides(values):
     np.testing.assert_array_equal(C, D)
 
 
+@pytest.mark.parametrize("scale", [1e-6, 1e-10, 1e-16])
+@pytest.mark.parametrize("values", ["counts", "positive", "normal"])
+def test_products_that_end_early(values, scale):
+    """PCFs of 1 to 400 elements that end, or change last, at a very early
+    time (walked in double precision up to there) and some whose last value
+    is not 0, among long ones."""
+    import stablebear_gb300 as sb
+    pts, off = _random(90, (1, 2, 33, 64, 400), values, seed=11)
+    for i in range(0, 90, 4):
+        a, b = int(off[i]), int(off[i + 1])
+        if i % 8 == 0:
+            pts[a:b, 0] *= scale
+        elif b - a > 2:
+            pts[a:a + 3, 0] *= scale
+            pts[a + 2:b, 1] = 0.0
+    X = sb.PcfArray.from_csr(pts, off)
+    _check(pts, off, sb.pdist(X).data, sb.pdist(X, p=2).data, sb.l2_kernel(X).data)
+    tails = pts.copy()
+    tails[np.asarray(off[1::9], dtype=np.int64) - 1, 1] = 2.0
+    X = sb.PcfArray.from_csr(tails, off)
+    from oracle import oracle as orc
+    want = orc.evaluate(tails, off, op=orc.OP_L2, mode=orc.MODE_KERNEL, truth=True)
+    ap = np.abs(tails)
+    bound = orc.evaluate(ap, off, op=orc.OP_L2, mode=orc.MODE_KERNEL, truth=True)
+    fine = np.isfinite(bound) & (bound < 1e300)
+    got = sb.l2_kernel(X).data
+    assert np.all(np.abs(got - want)[fine] <= TOL * bound[fine])
+
+
 def test_pairs_the_bound_refuses():
     """Near-identical PCFs, duplicates and functions that end at once: walked
     in double precision, or exactly 0."""
