@@ -25,7 +25,8 @@ namespace sbg
   };
 
   // A PCF's integer values (general form: over 2^32): sum of |changes|, of
-  // their squares, and the largest |value|.
+  // their squares, the largest |value|, and whether two different times of it
+  // (or one above 0 and 0) have the same integer (1, else 0).
   struct alignas(16) Shape { float tv, qv, vmax, close; };
 
   // One side's PCFs: CSR, processing order, and the packed arrays of `cap`
