@@ -779,7 +779,7 @@ namespace sbg
     struct FixedRun
     {
       int opk = 0, sms = 0;
-      uint32_t q = 1, smem = 0;
+      uint32_t q = 1, smem = 0, longest = 0;
       uint64_t rcap = 0, ccap = 0;
       bool cross = false;
       bool used[2] = {false, false};  // whose queue counters are no longer zero
@@ -814,6 +814,7 @@ namespace sbg
       {
         opk = opk_;
         sms = dev.sms;
+        longest = lmax;
         cross = mode == MODE_CROSS;
         rcap = std::max<uint64_t>(row_points, 1);
         ccap = cross ? std::max<uint64_t>(col_points, 1) : rcap;
@@ -833,7 +834,9 @@ namespace sbg
         cshape = cpack + up(ccap * 16);
         clens = cshape + up(nc * sizeof(Shape));
         carry = cross ? clens + up(nc * sizeof(uint32_t)) : cpack;
-        // one window takes every PCF, in the larger of the two element sizes
+        // one window takes every PCF, in the larger of the two element sizes:
+        // no sums pass from one to the next (a longer PCF than lmax does not
+        // get there, by the record)
         const uint32_t slots_bytes = (32 * q * 4 + 15) / 16 * 16;
         const bool one = lmax <= fixed_slice_cap(smem - slots_bytes, FIXED_WARPS, 16);
         carry_bytes = one ? 0 : up((size_t)sms * 32 * q * FIXED_CARRY * 32 * 8);
@@ -848,8 +851,8 @@ namespace sbg
       {
         base = at;
         SBG_CUDA(cudaMemsetAsync(base, 0, 256, st));
-        SBG_CUDA(launch_fixed_record(r.pts, r.off, r.n, rcap, record(), sms, st));
-        if (cross) SBG_CUDA(launch_fixed_record(c.pts, c.off, c.n, ccap, record(), sms, st));
+        SBG_CUDA(launch_fixed_record(r.pts, r.off, r.n, rcap, longest, record(), sms, st));
+        if (cross) SBG_CUDA(launch_fixed_record(c.pts, c.off, c.n, ccap, longest, record(), sms, st));
         SBG_CUDA(launch_fixed_pack(r.pts, r.off, r.n, rcap, record(), opk, rows(), row_shapes(), row_lens(), elements, gate(), sms, st));
         if (cross) SBG_CUDA(launch_fixed_pack(c.pts, c.off, c.n, ccap, record(), opk, cols(), col_shapes(), col_lens(), elements, gate(), sms, st));
         if (rperm) length_order_device(r.off, r.n, rperm, nullptr, st, row_lens());

@@ -99,10 +99,12 @@ namespace sbg
     }
 
     // One warp per PCF.  Times count from the second breakpoint on (the walk
-    // starts at 0 whatever the first says).
+    // starts at 0 whatever the first says).  A PCF longer than `longest`, which
+    // the host sized the call's buffers for, sends it to the direct kernels,
+    // which check lengths for themselves.
     __global__ void __launch_bounds__(256) fixed_record_kernel(const double* __restrict__ pts,
                                                                const uint64_t* __restrict__ off, uint64_t n,
-                                                               uint64_t cap, FixedRecord* rec)
+                                                               uint64_t cap, uint32_t longest, FixedRecord* rec)
     {
       const int lane = threadIdx.x & 31;
       const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -116,7 +118,7 @@ namespace sbg
       for (uint64_t i = w; i < n; i += nw)
       {
         const uint64_t o = off[i], e = off[i + 1];
-        if (e <= o || e > cap || e - o > 0xffffffffull) { bad = 1; continue; }
+        if (e <= o || e > cap || e - o > longest) { bad = 1; continue; }
         const uint64_t len = e - o;
         points += lane == 0 ? len : 0;
         for (uint64_t k = lane; k < len; k += 32)
@@ -953,12 +955,12 @@ namespace sbg
 
   // ---- launchers ----------------------------------------------------------------
 
-  cudaError_t launch_fixed_record(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap, FixedRecord* rec,
-                                  int sms, cudaStream_t st)
+  cudaError_t launch_fixed_record(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap, uint32_t longest,
+                                  FixedRecord* rec, int sms, cudaStream_t st)
   {
     if (n == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 8);
-    fixed_record_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, rec);
+    fixed_record_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, longest, rec);
     return launched();
   }
 

@@ -64,8 +64,9 @@ namespace sbg
     return (bytes - warps * 12 * elem) / (elem * (32 + warps)) / 4 * 4;
   }
 
-  cudaError_t launch_fixed_record(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap, FixedRecord* rec,
-                                  int sms, cudaStream_t st);
+  // longest: the breakpoint count that the call's buffers are sized for.
+  cudaError_t launch_fixed_record(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap, uint32_t longest,
+                                  FixedRecord* rec, int sms, cudaStream_t st);
   cudaError_t launch_fixed_pack(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
                                 const FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
                                 bool elements, unsigned* gate, int sms, cudaStream_t st);
