@@ -85,13 +85,17 @@ namespace sbg
 
     // Bin edges: quantiles of a sample of the breakpoint times, sorted in
     // shared memory by one CTA; edge 0 is time 0, edge `bins` the last time.
-    __global__ void __launch_bounds__(1024) l2_edges_kernel(const float* __restrict__ pts, uint64_t npts,
+    // Only points that the offsets cover: what stands behind them may be
+    // anything, and a NaN would leave the edges out of order.
+    __global__ void __launch_bounds__(1024) l2_edges_kernel(const float* __restrict__ pts,
+                                                            const uint64_t* __restrict__ off, uint64_t n,
                                                             const L2Record* __restrict__ rec, uint32_t bins,
                                                             float* __restrict__ edges)
     {
       __shared__ float s[SAMPLES];
       if (rec->bad) return;
-      for (uint32_t q = threadIdx.x; q < SAMPLES; q += 1024) s[q] = pts[2 * (uint64_t)((double)q * (double)npts / SAMPLES)];
+      const uint64_t o = off[0], covered = off[n] - o;
+      for (uint32_t q = threadIdx.x; q < SAMPLES; q += 1024) s[q] = pts[2 * (o + q * covered / SAMPLES)];
       // a stage at distance 32 or less stays within the 64 elements of a warp
       uint32_t before = 64;  // the loads cross warps
       for (uint32_t k = 2; k <= SAMPLES; k <<= 1)
@@ -831,7 +835,7 @@ namespace sbg
     SBG_CUDA(cudaMemsetAsync(base + p.record, 0, p.starts - p.record, st));  // the record and the counts
     l2_record_kernel<<<warps8, 256, 0, st>>>(pts, off, n, npts, rec);
     SBG_CUDA(launched());
-    l2_edges_kernel<<<1, 1024, 0, st>>>(pts, npts, rec, bins, f32(p.edges));
+    l2_edges_kernel<<<1, 1024, 0, st>>>(pts, off, n, rec, bins, f32(p.edges));
     SBG_CUDA(launched());
     auto u16 = [&](size_t at) { return reinterpret_cast<uint16_t*>(base + at); };
     uint64_t* keys = reinterpret_cast<uint64_t*>(base + p.keys);

@@ -1,0 +1,63 @@
+"""Data that the float32 L2 gradients by contraction (csrc/backward_l2.cu) must
+not be thrown off by, against the float64 gradients of the same numbers.
+
+Tolerance, as in test_gpu_l2_gradient.py: 2e-6 in the norm of the whole
+gradient, from about 600 rounded terms of random sign an entry."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 2e-6
+KINDS = ["kernel", "l2"]
+
+
+def _run(points, offsets, kind, w):
+    import torch
+    from stablebear_gb300 import autograd
+    P = points.clone().requires_grad_(True)
+    longest = int((offsets[1:] - offsets[:-1]).max())
+    f = autograd.l2_kernel if kind == "kernel" else autograd.pdist
+    out = f(P, offsets, max_points=longest)
+    grad, = torch.autograd.grad(out, P, w)
+    return out.detach(), grad
+
+
+def _data(n, lo, hi, seed):
+    import torch
+    rng = np.random.default_rng(seed)
+    ln = rng.integers(lo, hi + 1, n)
+    off = np.zeros(n + 1, np.int64)
+    np.cumsum(ln, out=off[1:])
+    t = np.concatenate([np.r_[0.0, np.cumsum(rng.exponential(1.0, k - 1) + 1e-3)] for k in ln])
+    v = rng.standard_normal(int(off[-1]))
+    v[off[1:] - 1] = 0.0
+    return torch.from_numpy(np.stack([t, v], 1).astype(np.float32)).cuda(), torch.from_numpy(off).cuda()
+
+
+def _weights(n, kind, seed):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return torch.randn(n * (n + 1) // 2 if kind == "kernel" else n * (n - 1) // 2, generator=g, device="cuda") / n
+
+
+def _near(got, want):
+    for c in range(2):
+        err = float((got[:, c].double() - want[:, c]).norm() / want[:, c].norm())
+        assert err <= TOL, (c, err)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rows", ["nan", "stale"])
+def test_rows_behind_the_last_pcf(kind, rows):
+    """A points tensor may be longer than the offsets say; what stands in the
+    rest is not read and gets no gradient."""
+    import torch
+    pts, off = _data(1000, 80, 150, seed=2)
+    spare = torch.full((len(pts) // 50, 2), float("nan") if rows == "nan" else -3e8, device="cuda")
+    both = torch.cat([pts, spare])
+    w = _weights(1000, kind, 2)
+    got = _run(both, off, kind, w)[1]
+    assert bool((got[len(pts):] == 0).all())
+    _near(got[:len(pts)], _run(pts.double(), off, kind, w.double())[1])
