@@ -27,7 +27,7 @@
 // Pairs that lie close together beside that are left to the walk (l2_close).
 //
 // A bin sum, a weight or a value that is not finite, a last value other than
-// 0 (its integral has no end) or times out of order make the walk of
+// 0 (its integral has no end) or times that do not ascend make the walk of
 // backward.cu run instead, decided by a record on the device.
 #include "sbg_internal.hpp"
 
@@ -48,7 +48,10 @@ namespace sbg
     constexpr int AHEAD = 4;            // list entries a lane has in flight
     constexpr uint32_t BIN_MAX = 8192;  // breakpoints of a bin
 
-    // Times from the second breakpoint on (the first is the start whatever it says).
+    // Times from the second breakpoint on (the first is the start whatever it
+    // says) have to ascend from above 0: at an element without width the walk
+    // gives the pair's row a time gradient and its column none.  That also
+    // keeps out -0, whose bits order above every other time's.
     __global__ void __launch_bounds__(256) l2_record_kernel(const float* __restrict__ pts,
                                                             const uint64_t* __restrict__ off, uint64_t n,
                                                             uint64_t npts, L2Record* rec)
@@ -69,7 +72,7 @@ namespace sbg
           if (k > 0)
           {
             const float t = pts[2 * (o + k)], before = k > 1 ? pts[2 * (o + k - 1)] : 0.0f;
-            bad |= !(t >= before) || !(t < FLT_MAX) ? 1u : 0u;
+            bad |= !(t > before) || !(t < FLT_MAX) ? 1u : 0u;
             tmax = max(tmax, __float_as_uint(t));
           }
         }

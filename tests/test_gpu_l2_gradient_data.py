@@ -61,3 +61,22 @@ def test_rows_behind_the_last_pcf(kind, rows):
     got = _run(both, off, kind, w)[1]
     assert bool((got[len(pts):] == 0).all())
     _near(got[:len(pts)], _run(pts.double(), off, kind, w.double())[1])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n,points", [(7500, 2), (1000, 120)])
+@pytest.mark.parametrize("where", ["zero", "negative zero", "twice"])
+def test_elements_without_width(kind, n, points, where):
+    """A breakpoint at time 0 (or -0.0) behind the first one, or two at one
+    time: an element without width, whose time gradient is the walk's.  7500
+    breakpoints fit one bin, 119,000 do not."""
+    pts, off = _data(n, points, points, seed=n)
+    k = off[:-1:7] + 1
+    if where == "twice":
+        if points < 3:
+            pytest.skip("needs a third breakpoint")
+        pts[k + 60, 0] = pts[k + 59, 0]
+    else:
+        pts[k, 0] = 0.0 if where == "zero" else -0.0
+    w = _weights(n, kind, 3)
+    _near(_run(pts, off, kind, w)[1], _run(pts.double(), off, kind, w.double())[1])
