@@ -26,9 +26,10 @@
 // differences count there, and sums of w_ij g_j then stay as small as them.
 // Pairs that lie close together beside that are left to the walk (l2_close).
 //
-// A bin sum, a weight or a value that is not finite, a last value other than
-// 0 (its integral has no end) or times that do not ascend make the walk of
-// backward.cu run instead, decided by a record on the device.
+// A weight or a value that is not finite, a last value other than 0 (its
+// integral has no end), times that do not ascend or a gradient that comes out
+// not finite make the walk of backward.cu run instead, decided by a record on
+// the device.
 #include "sbg_internal.hpp"
 
 #include "backward_l2.cuh"
@@ -523,7 +524,11 @@ namespace sbg
       __shared__ unsigned int s_bin;
       __shared__ float s_sum[ROWS_MAX];
       __shared__ uint32_t s_row[ROWS_MAX];
-      if (P.rec->bad | P.rec->bad_weights) return;
+      // bad_weights may be set by another CTA meanwhile: one answer for all threads
+      if (threadIdx.x == 0) s_bin = P.rec->bad | P.rec->bad_weights;
+      __syncthreads();
+      if (s_bin) return;
+      __syncthreads();
       const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = NEAR_THREADS / 32;
       const uint32_t n = (uint32_t)P.n;
       // Row r of group g is the (g + r groups)-th PCF in length order: the
@@ -559,6 +564,11 @@ namespace sbg
         }
         __syncthreads();
       }
+
+      // Some gradient is not finite.  A sum over all PCFs multiplies what
+      // overflows (one PCF's integral over a bin, say) by weights of 0 too,
+      // which the walk leaves out.
+      bool lost = false;
 
       // One breakpoint, from its bin's sums: H there, its time gradient, and
       // the integral of H from the bin's edge to it.
@@ -611,6 +621,7 @@ namespace sbg
           if (KERNEL) dt = fmaf(P.grad_out[i * (i + 1) / 2 + i], (a - c) * (a + c), dt);
           P.grad[2 * (o + k)] = dt;
           P.area[o + k] = fmaf(h0, t - edge, area);
+          lost |= !isfinite(dt);
         }
       };
 
@@ -743,8 +754,10 @@ namespace sbg
           if (KERNEL && !last) dv = fmaf(wii, 2.0f * (v * (t1 - t0)), dv);
           P.grad[2 * (o + k) + 1] = dv;
           if (k == 0) P.grad[2 * o] = 0.0f;
+          lost |= !isfinite(dv);
         }
       }
+      if (__any_sync(FULL, lost) && lane == 0) atomicOr(&P.rec->bad_weights, 1u);
     }
 
     uint64_t up(uint64_t x, uint64_t to) { return (x + to - 1) / to * to; }

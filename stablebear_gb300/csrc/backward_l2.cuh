@@ -6,8 +6,8 @@
 namespace sbg
 {
   // What the data of a call is like, gathered on the device (zeroed first).
-  // bad: the data takes the walk; bad_weights: a weight or an overfull bin
-  // does; close: some pairs of distances do (l2_close).
+  // bad: the data takes the walk; bad_weights: a weight, an overfull bin or a
+  // gradient that is not finite does; close: some pairs of distances do (l2_close).
   struct L2Record { uint32_t bad, bad_weights, close, tmax_bits; };
 
   // A distance far smaller than its two PCFs (less the common part): in
@@ -25,7 +25,7 @@ namespace sbg
 
   struct L2Gradient
   {
-    const L2Record* rec;
+    L2Record* rec;
     const float* pts;
     const uint64_t* off;
     const uint32_t* order;  // the PCFs in length order, panel by panel

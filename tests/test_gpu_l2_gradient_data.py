@@ -80,3 +80,25 @@ def test_elements_without_width(kind, n, points, where):
         pts[k, 0] = 0.0 if where == "zero" else -0.0
     w = _weights(n, kind, 3)
     _near(_run(pts, off, kind, w)[1], _run(pts.double(), off, kind, w.double())[1])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("size", [1e38, 3e38])
+def test_a_pcf_that_overflows(kind, size):
+    """One PCF whose integrals are beyond float32 and whose pairs all have
+    weight 0: it gets no gradient, and nobody gets one from it.  3e38: its
+    steps from value to value overflow too."""
+    import torch
+    n, one = 1000, 123
+    pts, off = _data(n, 80, 150, seed=7)
+    a, b = int(off[one]), int(off[one + 1])
+    pts[a:b - 1, 1] = size * torch.sign(pts[a:b - 1, 1])
+    w = torch.zeros(n, n, device="cuda")
+    i, j = torch.tril_indices(n, n, 0 if kind == "kernel" else -1, device="cuda")
+    w[i, j] = _weights(n, kind, 7)
+    w[one, :] = 0
+    w[:, one] = 0
+    w = w[i, j]
+    got = _run(pts, off, kind, w)[1]
+    assert bool((got[a:b] == 0).all())
+    _near(got, _run(pts.double(), off, kind, w.double())[1])
