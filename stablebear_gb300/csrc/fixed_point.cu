@@ -19,10 +19,11 @@
 //   general  |F| < 2^62; op(F, G) is the top 64 bits of the product, times
 //            the 62-bit width into a 128-bit sum.
 //
-// Error.  A time is off by at most half a unit, so a sum is off by at most
-// half the total change of op(F, G) along the merge, which the two PCFs'
-// variations bound; general values add at most two units of op per unit of
-// time.
+// Error.  A time of at least 2^52 units is a whole number of them, as is a
+// value of at least 2^52; a smaller one may be off by half a unit.  Each PCF
+// carries what that can move (Shape), and from two of those follows a bound of
+// the pair's error, whatever the order of its breakpoints and wherever its
+// windows end; op drops at most a unit per unit of time.
 // A pair whose bound is above 2^-47 of the sum of |terms| (the worst case of
 // the direct walk's naive blocks of 64) is walked again in double precision,
 // as is every pair of a call whose data fits no form (NaN or infinite values,
@@ -56,6 +57,15 @@ namespace sbg
       const int e = (int)(b >> 52);
       const uint64_t m = (b & 0xfffffffffffffull) | (e ? 1ull << 52 : 0ull);
       return (e ? e : 1) - 1075 + __ffsll((long long)m) - 1;
+    }
+    // Whether x 2^e is a whole number (x finite).
+    __device__ __forceinline__ bool whole(double x, int e)
+    {
+      const uint64_t b = (uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull;
+      const int field = (int)(b >> 52), low = field - 1075 + e;  // of the mantissa's last bit, scaled
+      if (b == 0 || (field && low >= 0)) return true;
+      if (field == 0 || low < -52) return false;
+      return (((b & 0xfffffffffffffull) | 1ull << 52) & ((1ull << -low) - 1)) == 0;
     }
     __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 
@@ -207,8 +217,7 @@ namespace sbg
                                k + 1 == len ? tmax_of<double>() : fmin(pts[2 * (o + k + 1)], tmax_of<double>())};
           continue;
         }
-        float tv = 0.0f, qv = 0.0f, vm = 0.0f;
-        bool close = false;  // two different times in one unit
+        float tv = 0.0f, ev = 0.0f, vm = 0.0f;
         uint64_t count = 0;  // elements before this chunk
         for (uint64_t k0 = 0; k0 < len; k0 += 32)
         {
@@ -221,11 +230,7 @@ namespace sbg
             if (k > 0)
             {
               before = pts[2 * (o + k) - 1];
-              const double u = k > 1 ? pts[2 * (o + k) - 2] : 0.0;
-              // (far apart by their high words but for the earliest times; the
-              // FP64 pipe is the slow one)
-              if (__double2hiint(t) - __double2hiint(u) < 2 || (__double2hiint(t) >> 20) < 1023 + 61 - f.s - 38)
-                close |= t > u && t * ts < 0x1p62 && __double2ll_rn(t * ts) == __double2ll_rn(u * ts);
+              if (f.kind == 2 && !whole(before, f.r)) ev += (float)((t - (k > 1 ? pts[2 * (o + k) - 2] : 0.0)) * ts);
             }
           }
           const bool starts = k < len && (k == 0 || v != before);
@@ -234,9 +239,7 @@ namespace sbg
           {
             const uint64_t at = o + count + __popc(mask & ((1u << lane) - 1u));  // <= o + k
             const long long F = __double2ll_rn(v * vs);
-            const float d = k == 0 ? 0.0f : fabsf((float)((v - before) * unit));
-            tv += d;
-            qv += d * d;
+            if (k > 0 && !whole(t, f.s)) tv += fabsf((float)((v - before) * unit));
             vm = fmaxf(vm, fabsf((float)F) * (f.kind == 1 ? 1.0f : 0x1p-32f));
             if (f.kind == 1)
               static_cast<uint32_t*>(values)[at] = (uint32_t)(int32_t)F;
@@ -256,15 +259,14 @@ namespace sbg
         for (int h = 16; h > 0; h >>= 1)
         {
           tv += __shfl_xor_sync(FULL, tv, h);
-          qv += __shfl_xor_sync(FULL, qv, h);
+          ev += __shfl_xor_sync(FULL, ev, h);
           vm = fmaxf(vm, __shfl_xor_sync(FULL, vm, h));
         }
-        const bool any_close = __any_sync(FULL, close);
         if (lane == 0)
         {
           times[o + count - 1] = f.kind == 1 ? ((T_END >> 31) << 32) | (T_END & 0x7fffffffull) : T_END;
           lens[i] = (uint32_t)count;
-          shapes[i] = Shape{tv, qv, vm, any_close ? 1.0f : 0.0f};
+          shapes[i] = Shape{tv, vm, ev, 0.0f};
         }
       }
     }
@@ -273,27 +275,25 @@ namespace sbg
 
     // Running sums of one lane's pair.
     //   add      one rectangle: op(F, G) = q, found before its side moved on
-    //   good     whether the error bound is within 2^-47 of the sum of |terms|
+    //   good     whether the error bound is within ACCEPT of the sum of |terms|
     //   value    the sum as a double, in units of time times op
     //
-    // Error of the times, in units of op.  Worst case: half the change of op
-    // along the merge, which the PCFs' own variation bounds (Shape), for the
-    // square by Cauchy-Schwarz: with no two breakpoints at once,
-    //   sum |q' - q| = sum |d' - d| |d' + d| <= 2 sqrt(sum (d' - d)^2 sum q).
-    // Or six standard deviations of independent roundings (each 1 / sqrt(12)
-    // of its change of op), where that is less.
+    // All of them are exact sums, the same however the pair was cut.
+    //
+    // The bound: with f' for f as rounded,
+    //   sum of |f' - f| over time <= f.tv / 2 + f.ev / 2   (times, then values),
+    // and op(f', g') - op(f, g) is at most
+    //   L1        |f' - f| + |g' - g|
+    //   products  |f' - f| max |g| + |g' - g| max |f|
+    //   squares   (|f' - f| + |g' - g|) 2 (max |f| + max |g|).
+    // (0.501 for a half: the floats here round.)
+    constexpr float ACCEPT = 0x1p-47f;
     template <int K>
-    __device__ __forceinline__ float time_error(const Shape& f, const Shape& g, float sum_q)
+    __device__ __forceinline__ float moved(const Shape& f, const Shape& g, float df, float dg)
     {
-      if (K == OPK_L1) return fminf(0.5f * (f.tv + g.tv), 1.75f * sqrtf(f.qv + g.qv));
-      if (K == OPK_INNER)
-        return fminf(0.5f * (f.vmax * g.tv + g.vmax * f.tv),
-                     1.75f * sqrtf(f.vmax * f.vmax * g.qv + g.vmax * g.vmax * f.qv));
-      // a window or row piece starts after the elements without width there,
-      // whose q is then not in the sum: where some are not without width
-      // before rounding, |d' + d| by the largest values
-      if (f.close + g.close > 0.0f) return (f.tv + g.tv) * (f.vmax + g.vmax);
-      return sqrtf(f.qv + g.qv) * sqrtf(sum_q);
+      if (K == OPK_L1) return 0.501f * (df + dg);
+      if (K == OPK_INNER) return 0.501f * (df * g.vmax + dg * f.vmax);
+      return 1.002f * (df + dg) * (f.vmax + g.vmax);
     }
 
     // Kept as 32-bit registers throughout: as 64-bit C++ variables the walk's
@@ -307,8 +307,7 @@ namespace sbg
       struct Q { int32_t q; };
       static constexpr uint32_t BYTES = 12;   // of an element in shared memory
       int64_t s0 = 0, s1 = 0;                 // sum = s1 2^31 + s0
-      uint64_t extra = 0;                     // L2: sum of q over the steps; signed products: sum of |q| times the high limb
-      uint32_t qs = 0;
+      int64_t a0 = 0, a1 = 0;                 // signed products: the same of |q|
 
       static __device__ __forceinline__ uint64_t end() { return ((T_END >> 31) << 32) | (T_END & 0x7fffffffull); }
       static __device__ __forceinline__ Q op(const Side& f, const Side& g)
@@ -325,31 +324,37 @@ namespace sbg
         const int32_t lo = (int32_t)(nl - tl), hi = (int32_t)(nh - th);
         s0 += (int64_t)q.q * lo;
         s1 += (int64_t)q.q * hi;
-        if (K == OPK_L2DIST) qs += (uint32_t)q.q;
-        if (SG) extra += (uint64_t)(uint32_t)abs(q.q) * (uint32_t)hi;
+        if (SG)
+        {
+          const int32_t a = abs(q.q);
+          a0 += (int64_t)a * lo;
+          a1 += (int64_t)a * hi;
+        }
       }
       __device__ __forceinline__ void block()  // s0 stays below 2^63 over a block's 8 steps of 2^28 * 2^31
       {
         s1 += s0 >> 31;
         s0 &= 0x7fffffff;
-        if (K == OPK_L2DIST)
+        if (SG)
         {
-          extra += qs;
-          qs = 0;
+          a1 += a0 >> 31;
+          a0 &= 0x7fffffff;
         }
       }
       __device__ __forceinline__ void save(uint64_t* c) const
       {
-        c[0] = (uint64_t)s0; c[32] = (uint64_t)s1; c[64] = extra;
+        c[0] = (uint64_t)s0; c[32] = (uint64_t)s1;
+        if (SG) { c[64] = (uint64_t)a0; c[96] = (uint64_t)a1; }
       }
       __device__ __forceinline__ void restore(const uint64_t* c)
       {
-        s0 = (int64_t)c[0]; s1 = (int64_t)c[32]; extra = c[64];
+        s0 = (int64_t)c[0]; s1 = (int64_t)c[32];
+        if (SG) { a0 = (int64_t)c[64]; a1 = (int64_t)c[96]; }
       }
       __device__ __forceinline__ bool good(const Shape& f, const Shape& g, uint64_t) const
       {
-        const float total = SG ? (float)extra : (float)s1;
-        return time_error<K>(f, g, (float)extra) * 0x1p47f <= total * 0x1p31f;
+        const float total = SG ? fmaf((float)a1, 0x1p31f, (float)a0) : fmaf((float)s1, 0x1p31f, (float)s0);
+        return moved<K>(f, g, f.tv, g.tv) <= total * ACCEPT;
       }
       __device__ __forceinline__ double value() const { return fma((double)s1, 0x1p31, (double)s0); }
       static __device__ __forceinline__ int scale(const Form& f) { return -f.s - (K == OPK_L1 ? f.r : 2 * f.r); }
@@ -362,9 +367,9 @@ namespace sbg
       struct Side { uint32_t lo, hi, v, w; };  // where the element ends, its value (low, high word)
       struct Q { uint32_t lo, hi, sign; };     // |op|, all ones where it is negative
       static constexpr uint32_t BYTES = 16;
-      uint32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;  // sum = s + h 2^64 + negatives
-      uint64_t h = 0, extra = 0;                // extra: as for Counts, of the high words
-      uint32_t negatives = 0;                   // terms subtracted as their one's complement
+      uint32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;  // sum of |terms| = s + h 2^64
+      uint64_t h = 0;
+      uint32_t n0 = 0, n1 = 0, n2 = 0, n3 = 0;  // signed products: that of the negative ones
 
       static __device__ __forceinline__ uint64_t end() { return T_END; }
       static __device__ __forceinline__ Q op(const Side& f, const Side& g)
@@ -407,10 +412,11 @@ namespace sbg
           const uint64_t t = (r >> 32) + (uint64_t)q.hi * bh;
           asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;"
               : "+r"(s0), "+r"(s1), "+r"(s2), "+r"(s3)
-              : "r"((uint32_t)p ^ q.sign), "r"((uint32_t)r ^ q.sign), "r"((uint32_t)t ^ q.sign),
-                "r"((uint32_t)(t >> 32) ^ q.sign));
-          negatives -= q.sign;
-          extra += (uint64_t)q.hi * bh;
+              : "r"((uint32_t)p), "r"((uint32_t)r), "r"((uint32_t)t), "r"((uint32_t)(t >> 32)));
+          asm("add.cc.u32 %0, %0, %4;\n\taddc.cc.u32 %1, %1, %5;\n\taddc.cc.u32 %2, %2, %6;\n\taddc.u32 %3, %3, %7;"
+              : "+r"(n0), "+r"(n1), "+r"(n2), "+r"(n3)
+              : "r"((uint32_t)p & q.sign), "r"((uint32_t)r & q.sign), "r"((uint32_t)t & q.sign),
+                "r"((uint32_t)(t >> 32) & q.sign));
         }
         else
         {
@@ -419,37 +425,47 @@ namespace sbg
               : "+r"(s0), "+r"(s1), "+r"(s2), "+r"(s3)
               : "r"((uint32_t)p), "r"((uint32_t)r), "r"((uint32_t)(r >> 32)));
         }
-        if (K == OPK_L2DIST) extra += q.hi;
       }
       __device__ __forceinline__ void block() { }
       __device__ __forceinline__ unsigned __int128 sum() const
       {
         const unsigned __int128 lo = ((uint64_t)s1 << 32) | s0, hi = (((uint64_t)s3 << 32) | s2) + h;
-        return (hi << 64) + lo + negatives;
+        return (hi << 64) + lo;
+      }
+      __device__ __forceinline__ unsigned __int128 negative() const
+      {
+        return ((unsigned __int128)(((uint64_t)n3 << 32) | n2) << 64) + (((uint64_t)n1 << 32) | n0);
       }
       __device__ __forceinline__ void save(uint64_t* c) const
       {
         const unsigned __int128 s = sum();
-        c[0] = (uint64_t)s; c[32] = (uint64_t)(s >> 64); c[64] = extra;
+        c[0] = (uint64_t)s; c[32] = (uint64_t)(s >> 64);
+        if (SG) { c[64] = ((uint64_t)n1 << 32) | n0; c[96] = ((uint64_t)n3 << 32) | n2; }
       }
       __device__ __forceinline__ void restore(const uint64_t* c)
       {
         s0 = (uint32_t)c[0]; s1 = (uint32_t)(c[0] >> 32);
         s2 = (uint32_t)c[32]; s3 = (uint32_t)(c[32] >> 32);
-        extra = c[64];
+        if (SG)
+        {
+          n0 = (uint32_t)c[64]; n1 = (uint32_t)(c[64] >> 32);
+          n2 = (uint32_t)c[96]; n3 = (uint32_t)(c[96] >> 32);
+        }
       }
-      // Shapes are in units of 2^32 here.  Besides the times: the values' own
-      // rounding and the dropped low word, two units of op over the time T of
-      // the later last breakpoint.
+      // Shapes' values are in units of 2^32 here, their times are not; products
+      // and squares are in units of 2^64 and drop up to one of those up to the
+      // time T of the later last breakpoint.
       __device__ __forceinline__ bool good(const Shape& f, const Shape& g, uint64_t T) const
       {
-        const float total = (float)(SG ? extra : (uint64_t)(sum() >> 64));  // in units of 2^64
-        const float times = time_error<K>(f, g, ((float)extra + 8192.0f) * 0x1p32f) * (K == OPK_L1 ? 0x1p32f : 1.0f);
-        return (times + (float)T * 2.0f) * 0x1p-17f <= total;
+        const unsigned __int128 s = sum();
+        const float total = fmaf((float)(uint64_t)(s >> 64), 0x1p64f, (float)(uint64_t)s);
+        const float times = moved<K>(f, g, f.tv, g.tv), values = moved<K>(f, g, f.ev, g.ev);
+        const float bound = K == OPK_L1 ? fmaf(times, 0x1p32f, values) : fmaf(values, 0x1p-32f, times) + (float)T;
+        return bound <= total * ACCEPT;
       }
       __device__ __forceinline__ double value() const
       {
-        const __int128 s = (__int128)sum();
+        const __int128 s = (__int128)(SG ? sum() - 2 * negative() : sum());
         const bool neg = SG && s < 0;
         const unsigned __int128 a = (unsigned __int128)(neg ? -s : s);
         const double v = fma((double)(uint64_t)(a >> 64), 0x1p64, (double)(uint64_t)a);

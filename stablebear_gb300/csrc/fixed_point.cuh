@@ -10,7 +10,7 @@ namespace sbg
   // values, N = 2500: 1.65 ms with 12 warps, 1.49 with 16, 1.57 with 20, 1.62
   // with 24).
   constexpr int FIXED_WARPS = 16;
-  constexpr uint32_t FIXED_CARRY = 3;  // 64-bit words of a pair's running sums
+  constexpr uint32_t FIXED_CARRY = 4;  // 64-bit words of a pair's running sums
 
   // What the data of a call is like, gathered on the device (zeroed first).
   struct FixedRecord
@@ -24,10 +24,10 @@ namespace sbg
     uint32_t pad;
   };
 
-  // A PCF's integer values (general form: over 2^32): sum of |changes|, of
-  // their squares, the largest |value|, and whether two different times of it
-  // (or one above 0 and 0) have the same integer (1, else 0).
-  struct alignas(16) Shape { float tv, qv, vmax, close; };
+  // What rounding can move of a PCF: the sum of |changes| at times that are no
+  // whole number of units, the largest |value| (both in integer values, general
+  // form: over 2^32), and for how long, in units, its value is no whole number.
+  struct alignas(16) Shape { float tv, vmax, ev, pad; };
 
   // One side's PCFs: CSR, processing order, and the packed arrays of `cap`
   // elements (times, then values).

@@ -61,3 +61,109 @@ def test_a_stated_length_below_the_longest(stated, longest, values):
         finally:
             sb.set_tuning()
         np.testing.assert_array_equal(got, want)
+
+
+# A pair whose error bound is above 2^-47 of its sum of |terms| is walked in
+# double precision (63 naive steps of 2^-53): both stay below 2^-46.
+TOL = 2.0 ** -46
+
+
+def _truth(rows, cols, p):
+    from oracle import oracle as orc
+    kw = dict(op=orc.OP_L1) if p == 1 else dict(op=orc.OP_LP, p=2.0)
+    out = orc.evaluate(rows[0], rows[1], col_points=cols[0], col_offsets=cols[1], mode=orc.MODE_CROSS, truth=True, **kw)
+    return out.reshape(len(rows[1]) - 1, len(cols[1]) - 1)
+
+
+def _join(lists):
+    off = np.zeros(len(lists) + 1, np.uint64)
+    np.cumsum([len(x) for x in lists], out=off[1:])
+    return np.concatenate(lists), off
+
+
+@pytest.mark.parametrize("values", ["counts", "normal"])
+def test_one_breakpoint_apart_by_less_than_a_unit(values):
+    """Pairs of steps that end apart by the last bit of a time, far below its
+    unit, at each of the 998 breakpoints of a long PCF that shares their
+    column group: where a time window ends there, the walk sees no difference."""
+    import stablebear_gb300 as sb
+    k = 1000
+    long, _ = _pcfs([k], values, seed=31)
+    long[-1, 0] = 2.0 ** 20 * long[-2, 0]
+    height = 3.0 if values == "counts" else float(np.pi)
+    rows, cols = [], []
+    for j in range(1, k - 1):
+        if len(cols) % 32 == 0:
+            cols.append(long)
+        t = long[j, 0]
+        rows.append(np.array([[0.0, height], [np.nextafter(t, np.inf), 0.0]]))
+        cols.append(np.array([[0.0, height], [t, 0.0]]))
+    steps = [i for i, c in enumerate(cols) if len(c) == 2]
+    rows, cols = _join(rows), _join(cols)
+    X, Y = sb.PcfArray.from_csr(*rows), sb.PcfArray.from_csr(*cols)
+    try:
+        sb.set_tuning(order=1)  # the groups as they are
+        got = [sb.cdist(X, Y, p=p) for p in (1, 2)]
+    finally:
+        sb.set_tuning()
+    for p in (1, 2):
+        want = _truth(rows, cols, p)[np.arange(k - 2), steps]
+        assert np.all(want > 0)
+        assert np.all(np.abs(got[p - 1][np.arange(k - 2), steps] - want) <= TOL * want), p
+
+
+def test_times_that_round_the_same_way():
+    """A falling staircase whose times all lie 0.4375 units behind a whole
+    one: their errors add up instead of evening out."""
+    import stablebear_gb300 as sb
+    steps = 4000
+    t = np.r_[0.0, np.arange(1, steps + 1) * 2.0 ** 33 + 0.4375]
+    stairs = np.stack([t, np.arange(steps, -1, -1.0)], 1)
+    rows = _join([stairs, np.array([[0.0, 1.0], [2.0 ** 61, 0.0]])])
+    cols = _join([np.zeros((1, 2)), np.array([[0.0, 1.0], [2.0 ** 43, 0.0]])])
+    X, Y = sb.PcfArray.from_csr(*rows), sb.PcfArray.from_csr(*cols)
+    for p in (1, 2):
+        want = _truth(rows, cols, p)
+        assert np.all(np.abs(sb.cdist(X, Y, p=p) - want) <= TOL * want), p
+
+
+@pytest.mark.parametrize("values", ["counts", "signed counts", "normal"])
+def test_long_and_close_pairs_do_not_depend_on_order_bands_or_sides(values):
+    """Which pairs are walked again is a matter of the pair alone: several
+    windows and row pieces, PCFs close together, early times below the unit."""
+    import stablebear_gb300 as sb
+    pts, off = _pcfs(np.random.default_rng(6).integers(400, 1500, 60), values, seed=6)
+    rng = np.random.default_rng(7)
+    lists = []
+    for i in range(60):
+        x = pts[int(off[i]):int(off[i + 1])].copy()
+        if i % 10 == 3:
+            x[:, 0] *= 0.01
+        lists.append(x)
+        for eps in (1e-3, 1e-7):
+            y = x.copy()
+            at = rng.integers(1, len(y) - 1, 5)
+            y[at, 0] = np.nextafter(y[at, 0], np.inf)
+            if values == "normal":
+                y[:-1, 1] += eps * rng.standard_normal(len(y) - 1)
+            lists.append(y)
+    lists[-1][-1, 0] *= 40.0  # the others' times below 2^56 units
+    lists += [np.array([[0.0, 1.0], [3.0, 0.0]])] * 900  # two processing-order windows
+    X = sb.PcfArray.from_csr(*_join(lists))
+    Y = X[:180]
+
+    def every():
+        return [sb.pdist(X).data.copy(), sb.pdist(X, p=2).data.copy(), sb.l2_kernel(X).data.copy(),
+                sb.cdist(Y, X).copy(), sb.cdist(Y, X, p=2).copy()]
+
+    try:
+        base = every()
+        for kw in (dict(order=1), dict(order=1, band_bytes=400 << 10), dict(band_bytes=400 << 10)):
+            sb.set_tuning(**kw)
+            for a, b in zip(every(), base):
+                np.testing.assert_array_equal(a, b)
+    finally:
+        sb.set_tuning()
+    for p, C in ((1, base[3]), (2, base[4])):
+        np.testing.assert_array_equal(sb.cdist(X, Y, p=p), C.T)
+        np.testing.assert_array_equal(sb.pdist(Y, p=p).to_dense(), C[:, :180])
