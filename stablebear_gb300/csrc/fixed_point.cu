@@ -310,6 +310,7 @@ namespace sbg
       int64_t a0 = 0, a1 = 0;                 // signed products: the same of |q|
 
       static __device__ __forceinline__ uint64_t end() { return ((T_END >> 31) << 32) | (T_END & 0x7fffffffull); }
+      static __device__ __forceinline__ uint64_t units(uint64_t t) { return ((t >> 32) << 31) | (t & 0x7fffffffull); }
       static __device__ __forceinline__ Q op(const Side& f, const Side& g)
       {
         // in asm: the compiler would widen the product to 64 bits
@@ -372,6 +373,7 @@ namespace sbg
       uint32_t n0 = 0, n1 = 0, n2 = 0, n3 = 0;  // signed products: that of the negative ones
 
       static __device__ __forceinline__ uint64_t end() { return T_END; }
+      static __device__ __forceinline__ uint64_t units(uint64_t t) { return t; }
       static __device__ __forceinline__ Q op(const Side& f, const Side& g)
       {
         if (K == OPK_INNER)  // magnitudes and signs: the top word of the product
@@ -914,7 +916,7 @@ namespace sbg
                 const double tail = op_f64<K>(rlast, clast);
                 if (tail != 0.0) res = fma(tail, tmax_of<double>(), res);
               }
-              const uint64_t Tr = rlen > 1 ? rtime[rlen - 2] : 0, Tc = clen > 1 ? ctime[clen - 2] : 0;
+              const uint64_t Tr = rlen > 1 ? A::units(rtime[rlen - 2]) : 0, Tc = clen > 1 ? A::units(ctime[clen - 2]) : 0;
               const Shape rshape = P.r.shapes[iorig];
               unsigned redo = __ballot_sync(FULL, ok && !acc.good(rshape, cshape, Tr > Tc ? Tr : Tc));
               while (redo)
