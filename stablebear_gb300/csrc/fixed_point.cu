@@ -584,18 +584,28 @@ namespace sbg
       return K == OPK_INNER ? f * g : K == OPK_L1 ? fabs(d) : d * d;
     }
 
-    // A pair in double precision, from the CSR points, by the whole warp: the
-    // longer PCF's elements split over the lanes, each lane's part walked in
-    // naive blocks of 64 rectangles under Kahan compensation, as the direct
-    // kernels sum, and the parts added.  (By the pair's own lane, its chain of
-    // dependent loads, one long row after the other, kept one SM busy for 23 ms
-    // at N = 1200: one column whose PCF ends at a very early time fails the
-    // test against every row.)
+    // A pair in double precision, from the CSR points: the longer PCF's
+    // elements in 32 parts, each walked in naive blocks of 64 rectangles under
+    // Kahan compensation, as the direct kernels sum, and the parts added
+    // neighbour to neighbour.  Few pairs of a row go one after the other, a
+    // part to a lane (one lane's chain of dependent loads would hold up the
+    // rest of the launch: 23 ms at N = 1200, where one column that ends early
+    // fails the test against every row); many go at once, a pair to a lane,
+    // part after part, with the same bits.  (Of 32 parts most lanes wait for
+    // the longest, and a part's start has to be searched for: N = 1000 near
+    // duplicates, L = 256, L2: 3.59 ms with the pairs at once, 7.95 one after
+    // the other, 2.48 in the direct kernel alone.)
+    //
     // Only what comes before `stop` counts, at or after the time from which
     // every term is 0 (the largest double: no such time): the products of a
     // PCF that ends early are over when it is, and the other's thousands of
     // later elements add nothing (the L2 kernel of 3500 stable ranks with a few
     // such: 2.98 ms with them, 0.98 without).
+    // Up to this many refused pairs of a row go one after the other (N = 1000,
+    // L = 256, one PCF ending 100 times later, the L2 kernel: 799 us with 16,
+    // 958 with 8, 960 with 4; L2 1056, 1059, 1170).
+    constexpr int MANY = 16;
+
     __device__ __forceinline__ uint32_t elements_before(const double* f, uint32_t n, double stop)
     {
       uint32_t lo = 1, hi = n;
@@ -606,87 +616,200 @@ namespace sbg
       }
       return lo;
     }
+
+    struct DirectPair
+    {
+      const double *f, *g;  // the longer one first
+      uint32_t nf, ng, per;
+      double stop;          // where both sides' last elements end
+
+      // Of equal lengths the one with the smaller first difference comes
+      // first, so that the sum does not depend on the pair's order.
+      template <int K, bool WARP>
+      __device__ __forceinline__ void set(const double* f_, uint32_t nf_, const double* g_, uint32_t ng_, double stop_)
+      {
+        f = f_; nf = nf_; g = g_; ng = ng_; stop = stop_;
+        if (K == OPK_INNER && stop < tmax_of<double>())
+        {
+          nf = elements_before(f, nf, stop);
+          ng = elements_before(g, ng, stop);
+        }
+        bool swap = nf < ng;
+        if (nf == ng)
+          for (uint32_t base = 0; base < nf; base += WARP ? 32 : 1)
+          {
+            const uint32_t k = WARP ? base + (threadIdx.x & 31) : base;
+            bool differ = false, more = false;
+            if (k < nf)
+            {
+              const double ft = k ? f[2 * k] : 0.0, gt = k ? g[2 * k] : 0.0, fv = f[2 * k + 1], gv = g[2 * k + 1];
+              differ = ft != gt || fv != gv;
+              more = ft > gt || (ft == gt && fv > gv);
+            }
+            if (WARP)
+            {
+              const unsigned m = __ballot_sync(FULL, differ);
+              if (!m) continue;
+              swap = __shfl_sync(FULL, more ? 1 : 0, __ffs((int)m) - 1) != 0;
+            }
+            else
+            {
+              if (!differ) continue;
+              swap = more;
+            }
+            break;
+          }
+        if (swap)
+        {
+          const double* p = f; f = g; g = p;
+          const uint32_t n = nf; nf = ng; ng = n;
+        }
+        per = (nf + 31) / 32;
+      }
+    };
+
+    // The sum over a part.
+    struct DirectSum
+    {
+      double acc = 0.0, comp = 0.0, blk = 0.0;
+      uint32_t k = 0;
+      __device__ __forceinline__ void flush()
+      {
+        const double y = blk - comp, s = acc + y;
+        comp = isfinite(s) ? (s - acc) - y : 0.0;
+        acc = s;
+        blk = 0.0;
+        k = 0;
+      }
+      __device__ __forceinline__ void add(double q, double width)
+      {
+        blk = fma(q, width, blk);
+        if (++k == 64) flush();
+      }
+      __device__ __forceinline__ double end()
+      {
+        if (k) flush();
+        const double x = acc - comp;
+        acc = comp = 0.0;
+        return x;
+      }
+    };
+
+    // Where the elements are read: point k's time and value, and the ones
+    // after the last, which never come.
+    struct DirectSide
+    {
+      const double* p;
+      uint32_t n, next;     // the point that `at` holds
+      double v, t, vn;      // the element's value, where it ends, the value after
+      double ta, va;        // the point behind that
+      double stop;
+      __device__ __forceinline__ void read()
+      {
+        const bool in = next < n;
+        ta = in ? p[2 * next] : stop;
+        va = in ? p[2 * next + 1] : 0.0;
+      }
+      __device__ __forceinline__ void start(const double* p_, uint32_t n_, uint32_t k, double stop_)
+      {
+        p = p_; n = n_; stop = stop_;
+        v = p[2 * k + 1];
+        next = k + 1;
+        read();
+        t = ta; vn = va;
+        ++next;
+        read();
+      }
+      __device__ __forceinline__ void advance()
+      {
+        v = vn; t = ta; vn = va;
+        ++next;
+        read();
+      }
+    };
+
+    // Parts [part, part + parts) of a pair, each handed to `done` with its sum.
+    template <int K, typename F>
+    __device__ __forceinline__ void direct_parts(const DirectPair& P, uint32_t part, uint32_t parts, F&& done)
+    {
+      uint32_t i = part * P.per;
+      if (i >= P.nf) return;
+      DirectSide f, g;
+      f.start(P.f, P.nf, i, P.stop);
+      uint32_t j = 0;
+      uint64_t t = i ? (uint64_t)__double_as_longlong(P.f[2 * i]) : 0;  // times >= 0 order as their bits
+      for (uint32_t lo = 1, hi = i ? P.ng : 1; lo < hi;)                // g's last breakpoint at or before t
+      {
+        const uint32_t mid = (lo + hi) / 2;
+        if ((uint64_t)__double_as_longlong(P.g[2 * mid]) <= t) { lo = mid + 1; j = mid; } else hi = mid;
+      }
+      g.start(P.g, P.ng, j, P.stop);
+      const uint64_t stop = (uint64_t)__double_as_longlong(P.stop);
+      uint32_t end = i + P.per;
+      DirectSum sum;
+      for (;;)
+      {
+        const uint64_t ft = (uint64_t)__double_as_longlong(f.t), gt = (uint64_t)__double_as_longlong(g.t);
+        const bool first = ft <= gt;
+        const uint64_t tn = first ? ft : gt;
+        if (tn != t)
+          sum.add(op_f64<K>(f.v, g.v), __longlong_as_double((long long)tn) - __longlong_as_double((long long)t));
+        t = tn;
+        if (first)
+        {
+          const bool over = tn == stop;  // both: f's end is not behind g's
+          ++i;
+          if (i == end || over)
+          {
+            done(part, sum.end());
+            ++part;
+            if (over || --parts == 0) break;
+            end += P.per;
+          }
+          f.advance();
+        }
+        else g.advance();
+      }
+    }
+
     template <int K>
     __device__ __noinline__ double direct_pair(const double* f, uint32_t nf, const double* g, uint32_t ng, double stop)
     {
-      const double TM = stop;  // where both sides' last elements end
-      if (K == OPK_INNER && stop < tmax_of<double>())
-      {
-        nf = elements_before(f, nf, stop);
-        ng = elements_before(g, ng, stop);
-      }
-      // the longer one first; of equal ones the one with the smaller first
-      // difference, so that the sum does not depend on the pair's order
-      const uint32_t lane = threadIdx.x & 31;
-      bool swap = nf < ng;
-      for (uint32_t base = 0; nf == ng && base < nf; base += 32)
-      {
-        const uint32_t k = base + lane;
-        bool differ = false, more = false;
-        if (k < nf)
-        {
-          const double ft = k ? f[2 * k] : 0.0, gt = k ? g[2 * k] : 0.0, fv = f[2 * k + 1], gv = g[2 * k + 1];
-          differ = ft != gt || fv != gv;
-          more = ft > gt || (ft == gt && fv > gv);
-        }
-        const unsigned m = __ballot_sync(FULL, differ);
-        if (m)
-        {
-          swap = __shfl_sync(FULL, more ? 1 : 0, __ffs((int)m) - 1) != 0;
-          break;
-        }
-      }
-      if (swap)
-      {
-        const double* p = f; f = g; g = p;
-        const uint32_t n = nf; nf = ng; ng = n;
-      }
-      const uint32_t per = (nf + 31) / 32, first = lane * per, end = min(nf, first + per);
-      double acc = 0.0;
-      if (first < end)
-      {
-        uint32_t i = first, j = 0;
-        double t = i ? f[2 * i] : 0.0;
-        for (uint32_t lo = 1, hi = ng; lo < hi;)  // the first of g's breakpoints after t
-        {
-          const uint32_t mid = (lo + hi) / 2;
-          if (g[2 * mid] <= t) { lo = mid + 1; j = mid; } else hi = mid;
-        }
-        double ft = i + 1 < nf ? f[2 * i + 2] : TM, gt = j + 1 < ng ? g[2 * j + 2] : TM, fv = f[2 * i + 1],
-               gv = g[2 * j + 1], comp = 0.0, blk = 0.0;
-        for (uint32_t k = 1;; ++k)
-        {
-          const double tn = ft <= gt ? ft : gt;
-          if (tn != t) blk = fma(op_f64<K>(fv, gv), tn - t, blk);
-          t = tn;
-          // a lane's part ends with its last element's own breakpoint
-          const bool done = ft <= gt && (i + 1 == end || (ft == TM && gt == TM));
-          if (k % 64 == 0 || done)
-          {
-            const double y = blk - comp, s = acc + y;
-            comp = isfinite(s) ? (s - acc) - y : 0.0;
-            acc = s;
-            blk = 0.0;
-          }
-          if (done) break;
-          if (ft <= gt)
-          {
-            ++i;
-            fv = f[2 * i + 1];
-            ft = i + 1 < nf ? f[2 * i + 2] : TM;
-          }
-          else
-          {
-            ++j;
-            gv = g[2 * j + 1];
-            gt = j + 1 < ng ? g[2 * j + 2] : TM;
-          }
-        }
-        acc -= comp;
-      }
+      DirectPair P;
+      P.set<K, true>(f, nf, g, ng, stop);
+      double x = 0.0;
+      direct_parts<K>(P, threadIdx.x & 31, 1, [&](uint32_t, double s) { x = s; });
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
-      return acc;
+      for (int o = 1; o < 32; o <<= 1) x += __shfl_xor_sync(FULL, x, o);
+      return x;
+    }
+
+    // The calling lane's own pair.
+    template <int K>
+    __device__ __noinline__ double direct_pair_of_lane(const double* f, uint32_t nf, const double* g, uint32_t ng,
+                                                       double stop)
+    {
+      DirectPair P;
+      P.set<K, false>(f, nf, g, ng, stop);
+      // sums of 2^l neighbours that wait for the next 2^l, as the lanes add
+      // them; parts that are not there are zeros
+      double wait[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, x = 0.0;
+      uint32_t n = 0;
+      auto push = [&](double s) {
+        bool carry = true;
+#pragma unroll
+        for (int l = 0; l < 5; ++l)
+          if (carry)
+          {
+            if (n >> l & 1) s = wait[l] + s;
+            else { wait[l] = s; carry = false; }
+          }
+        if (carry) x = s;
+        ++n;
+      };
+      direct_parts<K>(P, 0, 32, [&](uint32_t, double s) { push(s); });
+      while (n < 32) push(0.0);
+      return x;
     }
 
     // First k in [lo, hi] whose element of this lane's staged column ends
@@ -918,12 +1041,10 @@ namespace sbg
               }
               const uint64_t Tr = rlen > 1 ? A::units(rtime[rlen - 2]) : 0, Tc = clen > 1 ? A::units(ctime[clen - 2]) : 0;
               const Shape rshape = P.r.shapes[iorig];
-              unsigned redo = __ballot_sync(FULL, ok && !acc.good(rshape, cshape, Tr > Tc ? Tr : Tc));
-              while (redo)
+              const bool again = ok && !acc.good(rshape, cshape, Tr > Tc ? Tr : Tc);
+              unsigned redo = __ballot_sync(FULL, again);
+              if (redo)
               {
-                const int k = __ffs((int)redo) - 1;
-                redo &= redo - 1;
-                const uint64_t o = __shfl_sync(FULL, coff, k);
                 // the products' end, where a side's last value is 0: its last
                 // change, rounded up
                 uint64_t Te = ~0ull;
@@ -931,9 +1052,21 @@ namespace sbg
                 if (K == OPK_INNER && clast == 0.0) Te = Tc < Te ? Tc : Te;
                 const double stop =
                     Te == ~0ull ? tmax_of<double>() : ((double)Te + 1.0) * pow2(-form.s) * (1.0 + 0x1p-50);
-                const double x = direct_pair<K>(rpts, rpoints, P.c.pts + 2 * o, __shfl_sync(FULL, cpoints, k),
-                                                __shfl_sync(FULL, stop, k));
-                if (lane == k) res = x;
+                if (__popc(redo) > MANY)
+                {
+                  if (again) res = direct_pair_of_lane<K>(rpts, rpoints, P.c.pts + 2 * coff, cpoints, stop);
+                  __syncwarp();
+                }
+                else
+                  while (redo)
+                  {
+                    const int k = __ffs((int)redo) - 1;
+                    redo &= redo - 1;
+                    const uint64_t o = __shfl_sync(FULL, coff, k);
+                    const double x = direct_pair<K>(rpts, rpoints, P.c.pts + 2 * o, __shfl_sync(FULL, cpoints, k),
+                                                    __shfl_sync(FULL, stop, k));
+                    if (lane == k) res = x;
+                  }
               }
               if (ok)
               {

@@ -167,3 +167,42 @@ def test_long_and_close_pairs_do_not_depend_on_order_bands_or_sides(values):
     for p, C in ((1, base[3]), (2, base[4])):
         np.testing.assert_array_equal(sb.cdist(X, Y, p=p), C.T)
         np.testing.assert_array_equal(sb.pdist(Y, p=p).to_dense(), C[:, :180])
+
+
+@pytest.mark.parametrize("values", ["counts", "normal"])
+@pytest.mark.parametrize("k", [2, 3, 31, 33, 64, 65, 1000])
+def test_refused_pairs_alone_and_together(values, k):
+    """Pairs too close together, or ending too early, for the error bound: few
+    of a row are walked one after the other, a part to a lane, many at once, a
+    pair to a lane; with the same bits and within the tolerance."""
+    import stablebear_gb300 as sb
+    from oracle import oracle as orc
+    base, _ = _pcfs([k], values, seed=k)
+    rng = np.random.default_rng(k)
+    lists = []
+    for i in range(40):
+        x = base.copy()
+        x[:, 0] *= 2.0 ** -40  # all of it far below the unit of the last PCF's time
+        if i % 2 and k > 2:
+            x = np.delete(x, rng.integers(1, k - 1), axis=0)
+        x[1:, 0] *= 1 + 1e-9 * rng.random()
+        lists.append(x)
+    lists.append(np.array([[0.0, 1.0], [1e6, 0.0]]))
+    pts, off = _join(lists)
+    ap = np.abs(pts)
+    X = sb.PcfArray.from_csr(pts, off)
+    for name, got, kw in (("l1", sb.pdist(X).to_dense(), dict(op=orc.OP_L1, mode=orc.MODE_PDIST)),
+                          ("l2", sb.pdist(X, p=2).to_dense(), dict(op=orc.OP_LP, p=2.0, mode=orc.MODE_PDIST)),
+                          ("kernel", sb.l2_kernel(X).to_dense(), dict(op=orc.OP_L2, mode=orc.MODE_KERNEL))):
+        want = orc.evaluate(pts, off, truth=True, **kw)
+        scale = orc.evaluate(ap, off, truth=True, **kw) if name == "kernel" else want
+        i, j = np.tril_indices(41, 0 if name == "kernel" else -1)
+        assert np.all(np.abs(got[i, j] - want) <= TOL * scale), name
+        if name == "kernel":
+            continue
+        # the last PCF keeps the unit of time; a column group of three
+        for a in range(0, 40, 7):
+            few = sb.PcfArray.from_csr(*_join([lists[a], lists[(a + 11) % 40], lists[40]]))
+            C = sb.cdist(X, few, p=1 if name == "l1" else 2)
+            np.testing.assert_array_equal(C[:40, 0], got[:40, a])
+            np.testing.assert_array_equal(C[:40, 1], got[:40, (a + 11) % 40])
