@@ -108,6 +108,57 @@ namespace sbg
       return f;
     }
 
+    // ---- the error bound ------------------------------------------------------------
+    //
+    // With f' for f as rounded,
+    //   sum of |f' - f| over time <= f.tv / 2 + f.ev / 2   (times, then values),
+    // and op(f', g') - op(f, g) is at most
+    //   L1        |f' - f| + |g' - g|
+    //   products  |f' - f| max |g| + |g' - g| max |f|
+    //   squares   (|f' - f| + |g' - g|) 2 (max |f| + max |g|).
+    // (0.501 for a half: the floats here round.)  A pair is taken if that is
+    // within ACCEPT of its sum of |terms|.
+    constexpr float ACCEPT = 0x1p-47f;
+    __device__ __forceinline__ float moved(int opk, const Shape& f, const Shape& g, float df, float dg)
+    {
+      if (opk == OPK_L1) return 0.501f * (df + dg);
+      if (opk == OPK_INNER) return 0.501f * (df * g.vmax + dg * f.vmax);
+      return 1.002f * (df + dg) * (f.vmax + g.vmax);
+    }
+    __device__ __forceinline__ float counts_bound(int opk, const Shape& f, const Shape& g)
+    {
+      return moved(opk, f, g, f.tv, g.tv);
+    }
+    // Shapes' values are in units of 2^32 here, their times are not; products
+    // and squares are in units of 2^64 and drop up to one of those up to the
+    // time T of the later last breakpoint.
+    __device__ __forceinline__ float general_bound(int opk, const Shape& f, const Shape& g, float T)
+    {
+      const float times = moved(opk, f, g, f.tv, g.tv), values = moved(opk, f, g, f.ev, g.ev);
+      return opk == OPK_L1 ? fmaf(times, 0x1p32f, values) : fmaf(values, 0x1p-32f, times) + T;
+    }
+
+    // x 2^e as a float for estimates: cut off, not rounded, and 0 below 2^-126
+    // (without the FP64 pipe, which is the slow one).
+    __device__ __forceinline__ float scaled(double x, int e)
+    {
+      const int hi = __double2hiint(x), field = (hi >> 20 & 0x7ff) + e - 896;
+      if ((hi >> 20 & 0x7ff) == 0 || field < 1) return 0.0f;
+      return __uint_as_float((uint32_t)(hi & 0x80000000) | (uint32_t)min(field, 254) << 23 |
+                             (uint32_t)(hi & 0xfffff) << 3 | (uint32_t)__double2loint(x) >> 29);
+    }
+
+    // Whether the call had better go to the direct kernels at once: where most
+    // pairs would be refused, every pair would be walked twice.  A PCF is
+    // risky if a pair of it and one like it would be (fixed_pack_kernel);
+    // distances are refused where both sides are, products where one is.
+    // N = 1000, L = 256, one PCF ending 1000 times later, L1, L2, L2 kernel:
+    // REFUSE_US.
+    __device__ __forceinline__ bool mostly_refused(const FixedRecord& d, int opk)
+    {
+      return 10ull * d.risky > (opk == OPK_INNER ? 3ull : 7ull) * d.packed;
+    }
+
     // One warp per PCF.  Times count from the second breakpoint on (the walk
     // starts at 0 whatever the first says).  A PCF longer than `longest`, which
     // the host sized the call's buffers for, sends it to the direct kernels,
@@ -177,6 +228,15 @@ namespace sbg
       }
     }
 
+    // The (v, t) elements that the hybrid kernel reads, by a warp.
+    __device__ __forceinline__ void write_elements(const double* pts, uint64_t o, uint64_t len, Elem<double>* packed,
+                                                   int lane)
+    {
+      for (uint64_t k = lane; k < len; k += 32)
+        packed[o + k] = Elem<double>{pts[2 * (o + k) + 1],
+                                     k + 1 == len ? tmax_of<double>() : fmin(pts[2 * (o + k + 1)], tmax_of<double>())};
+    }
+
     // The times of a PCF's elements (an element ends where the value next
     // changes, the last at T_END) and their values, at the CSR's own offsets,
     // and how many there are: neighbours of equal value are one element (a
@@ -185,7 +245,7 @@ namespace sbg
     // kernel reads, in the same buffer, all of them.  One warp per PCF.
     __global__ void __launch_bounds__(256) fixed_pack_kernel(const double* __restrict__ pts,
                                                              const uint64_t* __restrict__ off, uint64_t n,
-                                                             uint64_t cap, const FixedRecord* __restrict__ rec, int opk,
+                                                             uint64_t cap, FixedRecord* rec, int opk,
                                                              void* __restrict__ packed, Shape* __restrict__ shapes,
                                                              uint32_t* __restrict__ lens, bool elements,
                                                              unsigned* __restrict__ gate)
@@ -198,6 +258,7 @@ namespace sbg
       uint64_t* times = static_cast<uint64_t*>(packed);
       void* values = times + cap;
       const double ts = pow2(f.s), vs = pow2(f.r), unit = pow2(f.kind == 1 ? f.r : f.r - 32);
+      uint32_t risky = 0, seen = 0;
       for (uint64_t i = w; i < n; i += nw)
       {
         const uint64_t o = off[i], e = off[i + 1];
@@ -210,14 +271,10 @@ namespace sbg
         if (f.kind == 0)
         {
           if (lane == 0) lens[i] = (uint32_t)len;
-          if (elements)
-            for (uint64_t k = lane; k < len; k += 32)
-              static_cast<Elem<double>*>(packed)[o + k] =
-                  Elem<double>{pts[2 * (o + k) + 1],
-                               k + 1 == len ? tmax_of<double>() : fmin(pts[2 * (o + k + 1)], tmax_of<double>())};
+          if (elements) write_elements(pts, o, len, static_cast<Elem<double>*>(packed), lane);
           continue;
         }
-        float tv = 0.0f, ev = 0.0f, vm = 0.0f;
+        float tv = 0.0f, ev = 0.0f, vm = 0.0f, area = 0.0f, end = 0.0f;
         uint64_t count = 0;  // elements before this chunk
         for (uint64_t k0 = 0; k0 < len; k0 += 32)
         {
@@ -230,7 +287,11 @@ namespace sbg
             if (k > 0)
             {
               before = pts[2 * (o + k) - 1];
-              if (f.kind == 2 && !whole(before, f.r)) ev += (float)((t - (k > 1 ? pts[2 * (o + k) - 2] : 0.0)) * ts);
+              const double u = k > 1 ? pts[2 * (o + k) - 2] : 0.0;
+              if (f.kind == 2 && !whole(before, f.r)) ev += (float)((t - u) * ts);
+              const float x = scaled(before, f.kind == 1 ? f.r : f.r - 32), at = scaled(t, f.s);
+              area = fmaf(opk == OPK_L1 ? fabsf(x) : x * x, at - scaled(u, f.s), area);
+              if (v != before) end = at;
             }
           }
           const bool starts = k < len && (k == 0 || v != before);
@@ -261,13 +322,26 @@ namespace sbg
           tv += __shfl_xor_sync(FULL, tv, h);
           ev += __shfl_xor_sync(FULL, ev, h);
           vm = fmaxf(vm, __shfl_xor_sync(FULL, vm, h));
+          area += __shfl_xor_sync(FULL, area, h);
+          end = fmaxf(end, __shfl_xor_sync(FULL, end, h));
         }
         if (lane == 0)
         {
           times[o + count - 1] = f.kind == 1 ? ((T_END >> 31) << 32) | (T_END & 0x7fffffffull) : T_END;
           lens[i] = (uint32_t)count;
-          shapes[i] = Shape{tv, vm, ev, 0.0f};
+          const Shape s{tv, vm, ev, 0.0f};
+          shapes[i] = s;
+          // a pair with one like it: |f - g| is about |f|, its square twice that of f
+          const float bound = f.kind == 1 ? counts_bound(opk, s, s) : general_bound(opk, s, s, end);
+          const float total = area * (opk == OPK_L2DIST ? 2.0f : opk == OPK_L1 && f.kind == 2 ? 0x1p32f : 1.0f);
+          risky += bound > total * ACCEPT ? 1u : 0u;
+          ++seen;
         }
+      }
+      if (lane == 0 && seen)
+      {
+        if (risky) atomicAdd(&rec->risky, risky);
+        atomicAdd(&rec->packed, seen);
       }
     }
 
@@ -279,23 +353,6 @@ namespace sbg
     //   value    the sum as a double, in units of time times op
     //
     // All of them are exact sums, the same however the pair was cut.
-    //
-    // The bound: with f' for f as rounded,
-    //   sum of |f' - f| over time <= f.tv / 2 + f.ev / 2   (times, then values),
-    // and op(f', g') - op(f, g) is at most
-    //   L1        |f' - f| + |g' - g|
-    //   products  |f' - f| max |g| + |g' - g| max |f|
-    //   squares   (|f' - f| + |g' - g|) 2 (max |f| + max |g|).
-    // (0.501 for a half: the floats here round.)
-    constexpr float ACCEPT = 0x1p-47f;
-    template <int K>
-    __device__ __forceinline__ float moved(const Shape& f, const Shape& g, float df, float dg)
-    {
-      if (K == OPK_L1) return 0.501f * (df + dg);
-      if (K == OPK_INNER) return 0.501f * (df * g.vmax + dg * f.vmax);
-      return 1.002f * (df + dg) * (f.vmax + g.vmax);
-    }
-
     // Kept as 32-bit registers throughout: as 64-bit C++ variables the walk's
     // tied asm operands and the products cost ten more instructions a step
     // (28 against 18 for counts).
@@ -355,7 +412,7 @@ namespace sbg
       __device__ __forceinline__ bool good(const Shape& f, const Shape& g, uint64_t) const
       {
         const float total = SG ? fmaf((float)a1, 0x1p31f, (float)a0) : fmaf((float)s1, 0x1p31f, (float)s0);
-        return moved<K>(f, g, f.tv, g.tv) <= total * ACCEPT;
+        return counts_bound(K, f, g) <= total * ACCEPT;
       }
       __device__ __forceinline__ double value() const { return fma((double)s1, 0x1p31, (double)s0); }
       static __device__ __forceinline__ int scale(const Form& f) { return -f.s - (K == OPK_L1 ? f.r : 2 * f.r); }
@@ -454,16 +511,11 @@ namespace sbg
           n2 = (uint32_t)c[96]; n3 = (uint32_t)(c[96] >> 32);
         }
       }
-      // Shapes' values are in units of 2^32 here, their times are not; products
-      // and squares are in units of 2^64 and drop up to one of those up to the
-      // time T of the later last breakpoint.
       __device__ __forceinline__ bool good(const Shape& f, const Shape& g, uint64_t T) const
       {
         const unsigned __int128 s = sum();
         const float total = fmaf((float)(uint64_t)(s >> 64), 0x1p64f, (float)(uint64_t)s);
-        const float times = moved<K>(f, g, f.tv, g.tv), values = moved<K>(f, g, f.ev, g.ev);
-        const float bound = K == OPK_L1 ? fmaf(times, 0x1p32f, values) : fmaf(values, 0x1p-32f, times) + (float)T;
-        return bound <= total * ACCEPT;
+        return general_bound(K, f, g, (float)T) <= total * ACCEPT;
       }
       __device__ __forceinline__ double value() const
       {
@@ -1086,11 +1138,35 @@ namespace sbg
       }
     }
 
+    // The hybrid kernel's (v, t) elements in the packed buffer, where the call
+    // turned out to be that kernel's.  One warp per PCF.
+    __global__ void __launch_bounds__(256) fixed_elements_kernel(const double* __restrict__ pts,
+                                                                 const uint64_t* __restrict__ off, uint64_t n,
+                                                                 uint64_t cap, const FixedRecord* __restrict__ rec,
+                                                                 int opk, Elem<double>* __restrict__ packed)
+    {
+      if (form_of(*rec, opk).kind == 0 || !mostly_refused(*rec, opk)) return;  // written already, or not needed
+      const int lane = threadIdx.x & 31;
+      const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+      const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+      for (uint64_t i = w; i < n; i += nw)
+      {
+        const uint64_t o = off[i], e = off[i + 1];
+        if (e <= o || e > cap) continue;
+        write_elements(pts, o, e - o, packed, lane);
+      }
+    }
+
     template <int K>
     __global__ void __launch_bounds__(FIXED_WARPS * 32, 1) fixed_pairs_kernel(const __grid_constant__ FixedParams P)
     {
       extern __shared__ __align__(16) unsigned char smem_raw[];
       const Form f = form_of(*P.rec, K);
+      if (f.kind != 0 && mostly_refused(*P.rec, K))
+      {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *P.gate = 0;  // opens the direct kernel behind this one
+        return;
+      }
       if (f.kind == 1)
       {
         if (K == OPK_INNER && f.sign) run_items<K, Counts<K, K == OPK_INNER>>(P, f, smem_raw);
@@ -1116,12 +1192,21 @@ namespace sbg
   }
 
   cudaError_t launch_fixed_pack(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
-                                const FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
+                                FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
                                 bool elements, unsigned* gate, int sms, cudaStream_t st)
   {
     if (n == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 8);
     fixed_pack_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, rec, opk, packed, shapes, lens, elements, gate);
+    return launched();
+  }
+
+  cudaError_t launch_fixed_elements(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
+                                    const FixedRecord* rec, int opk, void* packed, int sms, cudaStream_t st)
+  {
+    if (n == 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 8);
+    fixed_elements_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, rec, opk, static_cast<Elem<double>*>(packed));
     return launched();
   }
 

@@ -21,6 +21,8 @@ namespace sbg
     uint32_t low;                   // 4096 minus the exponent of the lowest bit set in any value
     uint32_t negative;              // some value is negative
     uint32_t bad;                   // not representable: the direct kernels run
+    uint32_t risky;                 // PCFs whose pairs would be walked twice, of
+    uint32_t packed;                // these many
     uint32_t pad;
   };
 
@@ -50,6 +52,7 @@ namespace sbg
     double* out;
     uint64_t out_base, out_count, ld, row_begin, row_end, n_items;
     unsigned long long* queue;  // zeroed before launch
+    unsigned* gate;             // of the direct kernel behind: 0 opens it
     uint64_t* carry;            // FIXED_CARRY * 32 words per row of an item and CTA
     uint32_t q, rows_per_item;
     int mode;
@@ -68,7 +71,9 @@ namespace sbg
   cudaError_t launch_fixed_record(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap, uint32_t longest,
                                   FixedRecord* rec, int sms, cudaStream_t st);
   cudaError_t launch_fixed_pack(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
-                                const FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
+                                FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
                                 bool elements, unsigned* gate, int sms, cudaStream_t st);
+  cudaError_t launch_fixed_elements(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
+                                    const FixedRecord* rec, int opk, void* packed, int sms, cudaStream_t st);
   cudaError_t launch_fixed_pairs(const FixedParams& P, int opk, int grid, cudaStream_t st);
 }

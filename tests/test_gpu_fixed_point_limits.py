@@ -206,3 +206,30 @@ def test_refused_pairs_alone_and_together(values, k):
             C = sb.cdist(X, few, p=1 if name == "l1" else 2)
             np.testing.assert_array_equal(C[:40, 0], got[:40, a])
             np.testing.assert_array_equal(C[:40, 1], got[:40, (a + 11) % 40])
+
+
+@pytest.mark.parametrize("values", ["counts", "signed counts", "normal"])
+@pytest.mark.parametrize("longest", [60, 300])
+def test_calls_whose_pairs_would_be_refused_take_the_direct_kernels(values, longest):
+    """One PCF that ends far behind the others takes the unit of time with it:
+    the direct kernels' bits (plain, then hybrid), also for two sets."""
+    import stablebear_gb300 as sb
+    lens = np.random.default_rng(longest).integers(20, longest, 70)
+    lens[0] = longest
+    pts, off = _pcfs(lens, values, seed=longest)
+    pts[int(off[6]) - 1, 0] *= 1e6
+    X = sb.PcfArray.from_csr(pts, off)
+    Y = X[:30]
+
+    def every():
+        return [sb.pdist(X).data.copy(), sb.pdist(X, p=2).data.copy(), sb.l2_kernel(X).data.copy(),
+                sb.cdist(X, Y).copy(), sb.cdist(Y, X, p=2).copy()]
+
+    got = every()
+    try:
+        sb.set_tuning(variant=5 if longest == 60 else 4)
+        want = every()
+    finally:
+        sb.set_tuning()
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
