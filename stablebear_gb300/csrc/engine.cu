@@ -855,11 +855,6 @@ namespace sbg
         if (cross) SBG_CUDA(launch_fixed_record(c.pts, c.off, c.n, ccap, longest, record(), sms, st));
         SBG_CUDA(launch_fixed_pack(r.pts, r.off, r.n, rcap, record(), opk, rows(), row_shapes(), row_lens(), elements, gate(), sms, st));
         if (cross) SBG_CUDA(launch_fixed_pack(c.pts, c.off, c.n, ccap, record(), opk, cols(), col_shapes(), col_lens(), elements, gate(), sms, st));
-        if (elements)
-        {
-          SBG_CUDA(launch_fixed_elements(r.pts, r.off, r.n, rcap, record(), opk, rows(), sms, st));
-          if (cross) SBG_CUDA(launch_fixed_elements(c.pts, c.off, c.n, ccap, record(), opk, cols(), sms, st));
-        }
         if (rperm) length_order_device(r.off, r.n, rperm, nullptr, st, row_lens());
         if (cross && cperm) length_order_device(c.off, c.n, cperm, nullptr, st, col_lens());
       }
@@ -879,6 +874,7 @@ namespace sbg
         P.rows_per_item = 32 * q;
         P.smem_bytes = smem;
         P.gate = gate();
+        P.elements = pl.packed;
         P.carry = reinterpret_cast<uint64_t*>(base + carry + (size_t)slot * carry_bytes);
         P.n_items = items_for(d.mode, d.row_begin, d.row_end, d.nc, q);
         if (P.n_items == 0) return;

@@ -152,8 +152,8 @@ namespace sbg
     // pairs would be refused, every pair would be walked twice.  A PCF is
     // risky if a pair of it and one like it would be (fixed_pack_kernel);
     // distances are refused where both sides are, products where one is.
-    // N = 1000, L = 256, one PCF ending 1000 times later, L1, L2, L2 kernel:
-    // REFUSE_US.
+    // N = 1000, L = 256, one PCF ending 1000 times later, L1 / L2 / L2 kernel:
+    // 1.89 / 2.50 / 1.89 ms, 9.42 / 10.1 / 9.74 with every pair walked twice.
     __device__ __forceinline__ bool mostly_refused(const FixedRecord& d, int opk)
     {
       return 10ull * d.risky > (opk == OPK_INNER ? 3ull : 7ull) * d.packed;
@@ -257,7 +257,8 @@ namespace sbg
       const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
       uint64_t* times = static_cast<uint64_t*>(packed);
       void* values = times + cap;
-      const double ts = pow2(f.s), vs = pow2(f.r), unit = pow2(f.kind == 1 ? f.r : f.r - 32);
+      const int unit_exp = f.kind == 1 ? f.r : f.r - 32;
+      const double ts = pow2(f.s), vs = pow2(f.r), unit = pow2(unit_exp);
       uint32_t risky = 0, seen = 0;
       for (uint64_t i = w; i < n; i += nw)
       {
@@ -287,11 +288,7 @@ namespace sbg
             if (k > 0)
             {
               before = pts[2 * (o + k) - 1];
-              const double u = k > 1 ? pts[2 * (o + k) - 2] : 0.0;
-              if (f.kind == 2 && !whole(before, f.r)) ev += (float)((t - u) * ts);
-              const float x = scaled(before, f.kind == 1 ? f.r : f.r - 32), at = scaled(t, f.s);
-              area = fmaf(opk == OPK_L1 ? fabsf(x) : x * x, at - scaled(u, f.s), area);
-              if (v != before) end = at;
+              if (f.kind == 2 && !whole(before, f.r)) ev += (float)((t - (k > 1 ? pts[2 * (o + k) - 2] : 0.0)) * ts);
             }
           }
           const bool starts = k < len && (k == 0 || v != before);
@@ -300,7 +297,13 @@ namespace sbg
           {
             const uint64_t at = o + count + __popc(mask & ((1u << lane) - 1u));  // <= o + k
             const long long F = __double2ll_rn(v * vs);
-            if (k > 0 && !whole(t, f.s)) tv += fabsf((float)((v - before) * unit));
+            if (k > 0)
+            {
+              if (!whole(t, f.s)) tv += fabsf((float)((v - before) * unit));
+              const float x = scaled(before, unit_exp), y = scaled(v, unit_exp);
+              end = scaled(t, f.s);
+              area = fmaf(opk == OPK_L1 ? fabsf(x) - fabsf(y) : (x - y) * (x + y), end, area);
+            }
             vm = fmaxf(vm, fabsf((float)F) * (f.kind == 1 ? 1.0f : 0x1p-32f));
             if (f.kind == 1)
               static_cast<uint32_t*>(values)[at] = (uint32_t)(int32_t)F;
@@ -824,44 +827,54 @@ namespace sbg
       }
     }
 
+    // The refused pairs of a row, bit l of `redo` for lane l's: this lane's
+    // integral, or `res` where it has none of them.  (One call, with all that
+    // only refused pairs need inside: two calls in the walk's loop cost it 2 %.)
     template <int K>
-    __device__ __noinline__ double direct_pair(const double* f, uint32_t nf, const double* g, uint32_t ng, double stop)
+    __device__ __noinline__ double walk_again(unsigned redo, const double* f, uint32_t nf, const double* g, uint32_t ng,
+                                              uint64_t end, int scale, double res)
     {
+      const uint32_t lane = threadIdx.x & 31;
+      const double stop = end == ~0ull ? tmax_of<double>() : ((double)end + 1.0) * pow2(-scale) * (1.0 + 0x1p-50);
       DirectPair P;
-      P.set<K, true>(f, nf, g, ng, stop);
-      double x = 0.0;
-      direct_parts<K>(P, threadIdx.x & 31, 1, [&](uint32_t, double s) { x = s; });
+      if (__popc(redo) > MANY)
+      {
+        if (!(redo >> lane & 1)) return res;
+        P.set<K, false>(f, nf, g, ng, stop);
+        // sums of 2^l neighbours that wait for the next 2^l, as the lanes add
+        // them below; parts that are not there are zeros
+        double wait[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        uint32_t n = 0;
+        auto push = [&](double s) {
+          bool carry = true;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) x += __shfl_xor_sync(FULL, x, o);
-      return x;
-    }
-
-    // The calling lane's own pair.
-    template <int K>
-    __device__ __noinline__ double direct_pair_of_lane(const double* f, uint32_t nf, const double* g, uint32_t ng,
-                                                       double stop)
-    {
-      DirectPair P;
-      P.set<K, false>(f, nf, g, ng, stop);
-      // sums of 2^l neighbours that wait for the next 2^l, as the lanes add
-      // them; parts that are not there are zeros
-      double wait[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, x = 0.0;
-      uint32_t n = 0;
-      auto push = [&](double s) {
-        bool carry = true;
+          for (int l = 0; l < 5; ++l)
+            if (carry)
+            {
+              if (n >> l & 1) s = wait[l] + s;
+              else { wait[l] = s; carry = false; }
+            }
+          if (carry) res = s;
+          ++n;
+        };
+        direct_parts<K>(P, 0, 32, [&](uint32_t, double s) { push(s); });
+        while (n < 32) push(0.0);
+        return res;
+      }
+      while (redo)
+      {
+        const int k = __ffs((int)redo) - 1;
+        redo &= redo - 1;
+        P.set<K, true>(f, nf, (const double*)__shfl_sync(FULL, (unsigned long long)g, k), __shfl_sync(FULL, ng, k),
+                       __shfl_sync(FULL, stop, k));
+        double x = 0.0;
+        direct_parts<K>(P, lane, 1, [&](uint32_t, double s) { x = s; });
+        __syncwarp();
 #pragma unroll
-        for (int l = 0; l < 5; ++l)
-          if (carry)
-          {
-            if (n >> l & 1) s = wait[l] + s;
-            else { wait[l] = s; carry = false; }
-          }
-        if (carry) x = s;
-        ++n;
-      };
-      direct_parts<K>(P, 0, 32, [&](uint32_t, double s) { push(s); });
-      while (n < 32) push(0.0);
-      return x;
+        for (int o = 1; o < 32; o <<= 1) x += __shfl_xor_sync(FULL, x, o);
+        if ((int)lane == k) res = x;
+      }
+      return res;
     }
 
     // First k in [lo, hi] whose element of this lane's staged column ends
@@ -1093,32 +1106,16 @@ namespace sbg
               }
               const uint64_t Tr = rlen > 1 ? A::units(rtime[rlen - 2]) : 0, Tc = clen > 1 ? A::units(ctime[clen - 2]) : 0;
               const Shape rshape = P.r.shapes[iorig];
-              const bool again = ok && !acc.good(rshape, cshape, Tr > Tc ? Tr : Tc);
-              unsigned redo = __ballot_sync(FULL, again);
+              const unsigned redo = __ballot_sync(FULL, ok && !acc.good(rshape, cshape, Tr > Tc ? Tr : Tc));
               if (redo)
               {
                 // the products' end, where a side's last value is 0: its last
                 // change, rounded up
-                uint64_t Te = ~0ull;
-                if (K == OPK_INNER && rlast == 0.0) Te = Tr;
-                if (K == OPK_INNER && clast == 0.0) Te = Tc < Te ? Tc : Te;
-                const double stop =
-                    Te == ~0ull ? tmax_of<double>() : ((double)Te + 1.0) * pow2(-form.s) * (1.0 + 0x1p-50);
-                if (__popc(redo) > MANY)
-                {
-                  if (again) res = direct_pair_of_lane<K>(rpts, rpoints, P.c.pts + 2 * coff, cpoints, stop);
-                  __syncwarp();
-                }
-                else
-                  while (redo)
-                  {
-                    const int k = __ffs((int)redo) - 1;
-                    redo &= redo - 1;
-                    const uint64_t o = __shfl_sync(FULL, coff, k);
-                    const double x = direct_pair<K>(rpts, rpoints, P.c.pts + 2 * o, __shfl_sync(FULL, cpoints, k),
-                                                    __shfl_sync(FULL, stop, k));
-                    if (lane == k) res = x;
-                  }
+                uint64_t end = ~0ull;
+                if (K == OPK_INNER && rlast == 0.0) end = Tr;
+                if (K == OPK_INNER && clast == 0.0) end = Tc < end ? Tc : end;
+                res = walk_again<K>(redo, rpts, rpoints, P.c.pts + 2 * coff, cpoints, end, form.s, res);
+                __syncwarp();
               }
               if (ok)
               {
@@ -1138,25 +1135,6 @@ namespace sbg
       }
     }
 
-    // The hybrid kernel's (v, t) elements in the packed buffer, where the call
-    // turned out to be that kernel's.  One warp per PCF.
-    __global__ void __launch_bounds__(256) fixed_elements_kernel(const double* __restrict__ pts,
-                                                                 const uint64_t* __restrict__ off, uint64_t n,
-                                                                 uint64_t cap, const FixedRecord* __restrict__ rec,
-                                                                 int opk, Elem<double>* __restrict__ packed)
-    {
-      if (form_of(*rec, opk).kind == 0 || !mostly_refused(*rec, opk)) return;  // written already, or not needed
-      const int lane = threadIdx.x & 31;
-      const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-      const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
-      for (uint64_t i = w; i < n; i += nw)
-      {
-        const uint64_t o = off[i], e = off[i + 1];
-        if (e <= o || e > cap) continue;
-        write_elements(pts, o, e - o, packed, lane);
-      }
-    }
-
     template <int K>
     __global__ void __launch_bounds__(FIXED_WARPS * 32, 1) fixed_pairs_kernel(const __grid_constant__ FixedParams P)
     {
@@ -1164,7 +1142,19 @@ namespace sbg
       const Form f = form_of(*P.rec, K);
       if (f.kind != 0 && mostly_refused(*P.rec, K))
       {
-        if (blockIdx.x == 0 && threadIdx.x == 0) *P.gate = 0;  // opens the direct kernel behind this one
+        // the direct kernel behind this one: its gate, and the elements it
+        // reads in the packed arrays' place (launches of other bands may do
+        // the same meanwhile, and write the same)
+        if (blockIdx.x == 0 && threadIdx.x == 0) *P.gate = 0;
+        if (!P.elements) return;
+        const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+        const uint64_t nw = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+        for (const FixedSet* s : {&P.r, &P.c})
+        {
+          if (s == &P.c && P.mode != MODE_CROSS) break;
+          for (uint64_t i = w; i < s->n; i += nw)
+            write_elements(s->pts, s->off[i], s->off[i + 1] - s->off[i], (Elem<double>*)s->times, threadIdx.x & 31);
+        }
         return;
       }
       if (f.kind == 1)
@@ -1198,15 +1188,6 @@ namespace sbg
     if (n == 0) return cudaSuccess;
     const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 8);
     fixed_pack_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, rec, opk, packed, shapes, lens, elements, gate);
-    return launched();
-  }
-
-  cudaError_t launch_fixed_elements(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
-                                    const FixedRecord* rec, int opk, void* packed, int sms, cudaStream_t st)
-  {
-    if (n == 0) return cudaSuccess;
-    const unsigned blocks = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 8);
-    fixed_elements_kernel<<<blocks, 256, 0, st>>>(pts, off, n, cap, rec, opk, static_cast<Elem<double>*>(packed));
     return launched();
   }
 

@@ -56,6 +56,7 @@ namespace sbg
     uint64_t* carry;            // FIXED_CARRY * 32 words per row of an item and CTA
     uint32_t q, rows_per_item;
     int mode;
+    bool elements;              // the direct kernel reads (v, t) elements in the packed arrays' place
     uint32_t smem_bytes;
   };
 
@@ -73,7 +74,5 @@ namespace sbg
   cudaError_t launch_fixed_pack(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
                                 FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
                                 bool elements, unsigned* gate, int sms, cudaStream_t st);
-  cudaError_t launch_fixed_elements(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
-                                    const FixedRecord* rec, int opk, void* packed, int sms, cudaStream_t st);
   cudaError_t launch_fixed_pairs(const FixedParams& P, int opk, int grid, cudaStream_t st);
 }
