@@ -814,7 +814,7 @@ namespace sbg
       {
         opk = opk_;
         sms = dev.sms;
-        longest = std::min(lmax, 0x7fffffffu);  // word indices into a PCF's points are 32-bit
+        longest = std::min(lmax, 0x3fffffffu);  // a pair's breakpoints and words are counted in 32 bits
         cross = mode == MODE_CROSS;
         rcap = std::max<uint64_t>(row_points, 1);
         ccap = cross ? std::max<uint64_t>(col_points, 1) : rcap;

@@ -16,22 +16,24 @@
 //            summaries are.  op(F, G) is an exact 32-bit integer; a rectangle
 //            costs two 32 x 32 -> 64 multiply-adds (times are kept as two
 //            31-bit limbs whose differences need no carry).
-//   general  |F| < 2^62; op(F, G) is the top 64 bits of the product, times
-//            the 62-bit width into a 128-bit sum.
+//   general  |F| < 2^62 (products: 2^63); op(F, G) is the top 64 bits of the
+//            product, times the 62-bit width into a 128-bit sum.
 //
 // Error.  A time of at least 2^52 units is a whole number of them, as is a
 // value of at least 2^52; a smaller one may be off by half a unit.  Each PCF
 // carries what that can move (Shape), and from two of those follows a bound of
 // the pair's error, whatever the order of its breakpoints and wherever its
 // windows end; op drops at most a unit per unit of time.
-// A pair whose bound is above 2^-47 of the sum of |terms| (the worst case of
-// the direct walk's naive blocks of 64) is walked again in double precision,
+// A pair whose usual error may be above 2^-51 of the sum of |terms|, or its
+// worst above 2^-47, is walked again in double precision,
 // as is every pair of a call whose data fits no form (NaN or infinite values,
 // times out of order, extreme exponents or outliers): then pairs_kernel or
 // the hybrid kernel runs instead, gated by the same device-side record.
 #include "sbg_internal.hpp"
 
 #include "fixed_point.cuh"
+
+#include <type_traits>
 
 namespace sbg
 {
@@ -104,7 +106,7 @@ namespace sbg
       const double mean = d.vsum / (double)(d.points ? d.points : 1);
       if (mean < vmax * (opk == OPK_L1 ? 0x1p-11 : 0x1p-6)) return f;
       f.kind = 2;
-      f.r = 61 - ve;
+      f.r = (opk == OPK_INNER ? 62 : 61) - ve;
       return f;
     }
 
@@ -116,26 +118,45 @@ namespace sbg
     //   L1        |f' - f| + |g' - g|
     //   products  |f' - f| max |g| + |g' - g| max |f|
     //   squares   (|f' - f| + |g' - g|) 2 (max |f| + max |g|).
-    // (0.501 for a half: the floats here round.)  A pair is taken if that is
-    // within ACCEPT of its sum of |terms|.
-    constexpr float ACCEPT = 0x1p-47f;
+    // (0.501 for a half: the floats here round.)  Roundings of times in both
+    // directions even out: usually a third of the root of the sum of squares
+    // stands for half the sum.  A pair is taken if its usual error is at most
+    // 2^-51 of its sum of |terms| (4.4e-16; the direct walk's is 3e-16), for
+    // squares 2^-50, which the root halves, and its worst at most 2^-47, the
+    // worst of the direct walk's naive blocks of 64.  Values count with their
+    // worst both times.
+    struct Bound
+    {
+      float worst, usual;
+      __device__ __forceinline__ bool within(int opk, float total) const
+      {
+        if (worst <= total * 0x1p-51f) return true;  // most pairs
+        return worst <= total * 0x1p-47f && usual <= total * (opk == OPK_L2DIST ? 0x1p-50f : 0x1p-51f);
+      }
+    };
     __device__ __forceinline__ float moved(int opk, const Shape& f, const Shape& g, float df, float dg)
     {
       if (opk == OPK_L1) return 0.501f * (df + dg);
       if (opk == OPK_INNER) return 0.501f * (df * g.vmax + dg * f.vmax);
       return 1.002f * (df + dg) * (f.vmax + g.vmax);
     }
-    __device__ __forceinline__ float counts_bound(int opk, const Shape& f, const Shape& g)
+    __device__ __forceinline__ Bound counts_bound(int opk, const Shape& f, const Shape& g)
     {
-      return moved(opk, f, g, f.tv, g.tv);
+      // (products of general values are beyond a float when squared)
+      const float a = opk == OPK_INNER ? f.rv * 0x1p-20f * (g.vmax * 0x1p-20f) : f.rv;
+      const float b = opk == OPK_INNER ? g.rv * 0x1p-20f * (f.vmax * 0x1p-20f) : g.rv;
+      const float scale = opk == OPK_L1 ? 1.0f : opk == OPK_INNER ? 0x1p40f : 2.0f * (f.vmax + g.vmax);
+      return Bound{moved(opk, f, g, f.tv, g.tv), 0.289f * sqrtf(fmaf(a, a, b * b)) * scale};
     }
     // Shapes' values are in units of 2^32 here, their times are not; products
     // and squares are in units of 2^64 and drop up to one of those up to the
-    // time T of the later last breakpoint.
-    __device__ __forceinline__ float general_bound(int opk, const Shape& f, const Shape& g, float T)
+    // time T from which they are 0.
+    __device__ __forceinline__ Bound general_bound(int opk, const Shape& f, const Shape& g, float T)
     {
-      const float times = moved(opk, f, g, f.tv, g.tv), values = moved(opk, f, g, f.ev, g.ev);
-      return opk == OPK_L1 ? fmaf(times, 0x1p32f, values) : fmaf(values, 0x1p-32f, times) + T;
+      const Bound t = counts_bound(opk, f, g);
+      const float v = moved(opk, f, g, f.ev, g.ev);
+      if (opk == OPK_L1) return Bound{fmaf(t.worst, 0x1p32f, v), fmaf(t.usual, 0x1p32f, v)};
+      return Bound{fmaf(v, 0x1p-32f, t.worst) + T, fmaf(v, 0x1p-32f, t.usual) + T};
     }
 
     // x 2^e as a float for estimates: cut off, not rounded, and 0 below 2^-126
@@ -156,7 +177,7 @@ namespace sbg
     // 1.89 / 2.50 / 1.89 ms, 9.42 / 10.1 / 9.74 with every pair walked twice.
     __device__ __forceinline__ bool mostly_refused(const FixedRecord& d, int opk)
     {
-      return 10ull * d.risky > (opk == OPK_INNER ? 3ull : 7ull) * d.packed;
+      return 10ull * d.risky > (opk == OPK_INNER ? 2ull : 7ull) * d.packed;
     }
 
     // One warp per PCF.  Times count from the second breakpoint on (the walk
@@ -275,7 +296,7 @@ namespace sbg
           if (elements) write_elements(pts, o, len, static_cast<Elem<double>*>(packed), lane);
           continue;
         }
-        float tv = 0.0f, ev = 0.0f, vm = 0.0f, area = 0.0f, end = 0.0f;
+        float tv = 0.0f, qv = 0.0f, ev = 0.0f, vm = 0.0f, area = 0.0f, end = 0.0f;
         uint64_t count = 0;  // elements before this chunk
         for (uint64_t k0 = 0; k0 < len; k0 += 32)
         {
@@ -299,7 +320,12 @@ namespace sbg
             const long long F = __double2ll_rn(v * vs);
             if (k > 0)
             {
-              if (!whole(t, f.s)) tv += fabsf((float)((v - before) * unit));
+              if (!whole(t, f.s))
+              {
+                const float c = fabsf((float)((v - before) * unit));
+                tv += c;
+                qv = fmaf(c, c, qv);
+              }
               const float x = scaled(before, unit_exp), y = scaled(v, unit_exp);
               end = scaled(t, f.s);
               area = fmaf(opk == OPK_L1 ? fabsf(x) - fabsf(y) : (x - y) * (x + y), end, area);
@@ -323,6 +349,7 @@ namespace sbg
         for (int h = 16; h > 0; h >>= 1)
         {
           tv += __shfl_xor_sync(FULL, tv, h);
+          qv += __shfl_xor_sync(FULL, qv, h);
           ev += __shfl_xor_sync(FULL, ev, h);
           vm = fmaxf(vm, __shfl_xor_sync(FULL, vm, h));
           area += __shfl_xor_sync(FULL, area, h);
@@ -332,12 +359,13 @@ namespace sbg
         {
           times[o + count - 1] = f.kind == 1 ? ((T_END >> 31) << 32) | (T_END & 0x7fffffffull) : T_END;
           lens[i] = (uint32_t)count;
-          const Shape s{tv, vm, ev, 0.0f};
+          const Shape s{tv, vm, ev, sqrtf(qv)};
           shapes[i] = s;
-          // a pair with one like it: |f - g| is about |f|, its square twice that of f
-          const float bound = f.kind == 1 ? counts_bound(opk, s, s) : general_bound(opk, s, s, end);
-          const float total = area * (opk == OPK_L2DIST ? 2.0f : opk == OPK_L1 && f.kind == 2 ? 0x1p32f : 1.0f);
-          risky += bound > total * ACCEPT ? 1u : 0u;
+          // a pair with one like it: |f - g| is about |f|, its square twice that
+          // of f, |f g| some five eighths of it
+          const Bound bound = f.kind == 1 ? counts_bound(opk, s, s) : general_bound(opk, s, s, end);
+          const float total = area * (opk == OPK_L2DIST ? 2.0f : opk == OPK_INNER ? 0.625f : f.kind == 2 ? 0x1p32f : 1.0f);
+          risky += bound.within(opk, total) ? 0u : 1u;
           ++seen;
         }
       }
@@ -352,7 +380,7 @@ namespace sbg
 
     // Running sums of one lane's pair.
     //   add      one rectangle: op(F, G) = q, found before its side moved on
-    //   good     whether the error bound is within ACCEPT of the sum of |terms|
+    //   good     whether the error bound is small enough against the sum of |terms|
     //   value    the sum as a double, in units of time times op
     //
     // All of them are exact sums, the same however the pair was cut.
@@ -366,6 +394,7 @@ namespace sbg
       struct Side { uint32_t lo, hi, v; };    // where the element ends (two 31-bit limbs), its value
       struct Q { int32_t q; };
       static constexpr uint32_t BYTES = 12;   // of an element in shared memory
+      static constexpr bool DROPS = false;    // whether op drops part of a unit
       int64_t s0 = 0, s1 = 0;                 // sum = s1 2^31 + s0
       int64_t a0 = 0, a1 = 0;                 // signed products: the same of |q|
 
@@ -415,7 +444,7 @@ namespace sbg
       __device__ __forceinline__ bool good(const Shape& f, const Shape& g, uint64_t) const
       {
         const float total = SG ? fmaf((float)a1, 0x1p31f, (float)a0) : fmaf((float)s1, 0x1p31f, (float)s0);
-        return counts_bound(K, f, g) <= total * ACCEPT;
+        return counts_bound(K, f, g).within(K, total);
       }
       __device__ __forceinline__ double value() const { return fma((double)s1, 0x1p31, (double)s0); }
       static __device__ __forceinline__ int scale(const Form& f) { return -f.s - (K == OPK_L1 ? f.r : 2 * f.r); }
@@ -428,6 +457,7 @@ namespace sbg
       struct Side { uint32_t lo, hi, v, w; };  // where the element ends, its value (low, high word)
       struct Q { uint32_t lo, hi, sign; };     // |op|, all ones where it is negative
       static constexpr uint32_t BYTES = 16;
+      static constexpr bool DROPS = K != OPK_L1;
       uint32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0;  // sum of |terms| = s + h 2^64
       uint64_t h = 0;
       uint32_t n0 = 0, n1 = 0, n2 = 0, n3 = 0;  // signed products: that of the negative ones
@@ -518,7 +548,7 @@ namespace sbg
       {
         const unsigned __int128 s = sum();
         const float total = fmaf((float)(uint64_t)(s >> 64), 0x1p64f, (float)(uint64_t)s);
-        return general_bound(K, f, g, (float)T) <= total * ACCEPT;
+        return general_bound(K, f, g, (float)T).within(K, total);
       }
       __device__ __forceinline__ double value() const
       {
@@ -639,87 +669,50 @@ namespace sbg
       return K == OPK_INNER ? f * g : K == OPK_L1 ? fabs(d) : d * d;
     }
 
-    // A pair in double precision, from the CSR points: the longer PCF's
-    // elements in 32 parts, each walked in naive blocks of 64 rectangles under
-    // Kahan compensation, as the direct kernels sum, and the parts added
-    // neighbour to neighbour.  Few pairs of a row go one after the other, a
-    // part to a lane (one lane's chain of dependent loads would hold up the
-    // rest of the launch: 23 ms at N = 1200, where one column that ends early
-    // fails the test against every row); many go at once, a pair to a lane,
-    // part after part, with the same bits.  (Of 32 parts most lanes wait for
-    // the longest, and a part's start has to be searched for: N = 1000 near
-    // duplicates, L = 256, L2: 3.59 ms with the pairs at once, 7.95 one after
-    // the other, 2.48 in the direct kernel alone.)
+    // A pair in double precision, from the CSR points: the merged breakpoints
+    // of both in 32 parts of equal number, each walked in naive blocks of 64
+    // rectangles under Kahan compensation, as the direct kernels sum, and the
+    // parts added neighbour to neighbour.  Nothing in that depends on which PCF
+    // comes first.  Few pairs of a row go one after the other, a part to a lane
+    // (one lane's chain of dependent loads would hold up the rest of the launch:
+    // 23 ms at N = 1200, where one column that ends early fails the test against
+    // every row); many go at once, a pair to a lane, part after part, with the
+    // same bits (N = 1000 near duplicates, L = 256, L2: 3.60 ms with the pairs
+    // at once, 7.95 one after the other, 2.48 in the direct kernel alone).
     //
     // Only what comes before `stop` counts, at or after the time from which
     // every term is 0 (the largest double: no such time): the products of a
     // PCF that ends early are over when it is, and the other's thousands of
     // later elements add nothing (the L2 kernel of 3500 stable ranks with a few
     // such: 2.98 ms with them, 0.98 without).
-    // Up to this many refused pairs of a row go one after the other (N = 1000,
-    // L = 256, one PCF ending 100 times later, the L2 kernel: 799 us with 16,
-    // 958 with 8, 960 with 4; L2 1056, 1059, 1170).
-    constexpr int MANY = 16;
-
     __device__ __forceinline__ uint32_t elements_before(const double* f, uint32_t n, double stop)
     {
       uint32_t lo = 1, hi = n;
       while (lo < hi)
       {
         const uint32_t mid = (lo + hi) / 2;
-        if (f[2 * (uint64_t)mid] < stop) lo = mid + 1; else hi = mid;
+        if (f[2 * mid] < stop) lo = mid + 1; else hi = mid;
       }
       return lo;
     }
 
     struct DirectPair
     {
-      const double *f, *g;  // the longer one first
-      uint32_t nf, ng, per;
-      double stop;          // where both sides' last elements end
+      const double *f, *g;
+      uint32_t nf, ng, per;  // elements; breakpoints of a part, the end at `stop` one of them
+      double stop;           // where both sides' last elements end
 
-      // Of equal lengths the one with the smaller first difference comes
-      // first, so that the sum does not depend on the pair's order.
-      template <int K, bool WARP>
-      __device__ __forceinline__ void set(const double* f_, uint32_t nf_, const double* g_, uint32_t ng_, double stop_)
+      template <int K>
+      __device__ __forceinline__ DirectPair(const double* f_, uint32_t nf_, const double* g_, uint32_t ng_,
+                                            double stop_, std::integral_constant<int, K>)
+          : f(f_), g(g_), nf(nf_), ng(ng_), stop(stop_)
       {
-        f = f_; nf = nf_; g = g_; ng = ng_; stop = stop_;
         if (K == OPK_INNER && stop < tmax_of<double>())
         {
           nf = elements_before(f, nf, stop);
           ng = elements_before(g, ng, stop);
         }
-        bool swap = nf < ng;
-        if (nf == ng)
-          for (uint32_t base = 0; base < nf; base += WARP ? 32 : 1)
-          {
-            const uint32_t k = WARP ? base + (threadIdx.x & 31) : base;
-            bool differ = false, more = false;
-            if (k < nf)
-            {
-              const double ft = k ? f[2 * k] : 0.0, gt = k ? g[2 * k] : 0.0, fv = f[2 * k + 1], gv = g[2 * k + 1];
-              differ = ft != gt || fv != gv;
-              more = ft > gt || (ft == gt && fv > gv);
-            }
-            if (WARP)
-            {
-              const unsigned m = __ballot_sync(FULL, differ);
-              if (!m) continue;
-              swap = __shfl_sync(FULL, more ? 1 : 0, __ffs((int)m) - 1) != 0;
-            }
-            else
-            {
-              if (!differ) continue;
-              swap = more;
-            }
-            break;
-          }
-        if (swap)
-        {
-          const double* p = f; f = g; g = p;
-          const uint32_t n = nf; nf = ng; ng = n;
-        }
-        per = (nf + 31) / 32;
+        per = (nf + ng - 1 + 31) / 32;
       }
     };
 
@@ -787,22 +780,25 @@ namespace sbg
     template <int K, typename F>
     __device__ __forceinline__ void direct_parts(const DirectPair& P, uint32_t part, uint32_t parts, F&& done)
     {
-      uint32_t i = part * P.per;
-      if (i >= P.nf) return;
+      const uint32_t d = part * P.per;  // breakpoints before the first part
+      if (d >= P.nf + P.ng - 1) return;
+      // i of them are f's, j are g's
+      uint32_t i = d > P.ng - 1 ? d - (P.ng - 1) : 0;
+      for (uint32_t hi = min(d, P.nf - 1); i < hi;)
+      {
+        const uint32_t mid = (i + hi) / 2;
+        if (P.f[2 * (mid + 1)] <= P.g[2 * (d - mid)]) i = mid + 1; else hi = mid;
+      }
+      const uint32_t j = d - i;
+      // times >= 0 order as their bits
+      uint64_t t = i ? (uint64_t)__double_as_longlong(P.f[2 * i]) : 0;
+      if (j) t = max(t, (uint64_t)__double_as_longlong(P.g[2 * j]));
       DirectSide f, g;
       f.start(P.f, P.nf, i, P.stop);
-      uint32_t j = 0;
-      uint64_t t = i ? (uint64_t)__double_as_longlong(P.f[2 * i]) : 0;  // times >= 0 order as their bits
-      for (uint32_t lo = 1, hi = i ? P.ng : 1; lo < hi;)                // g's last breakpoint at or before t
-      {
-        const uint32_t mid = (lo + hi) / 2;
-        if ((uint64_t)__double_as_longlong(P.g[2 * mid]) <= t) { lo = mid + 1; j = mid; } else hi = mid;
-      }
       g.start(P.g, P.ng, j, P.stop);
       const uint64_t stop = (uint64_t)__double_as_longlong(P.stop);
-      uint32_t end = i + P.per;
       DirectSum sum;
-      for (;;)
+      for (uint32_t k = 1;; ++k)
       {
         const uint64_t ft = (uint64_t)__double_as_longlong(f.t), gt = (uint64_t)__double_as_longlong(g.t);
         const bool first = ft <= gt;
@@ -810,20 +806,13 @@ namespace sbg
         if (tn != t)
           sum.add(op_f64<K>(f.v, g.v), __longlong_as_double((long long)tn) - __longlong_as_double((long long)t));
         t = tn;
-        if (first)
+        if (k == P.per || tn == stop)
         {
-          const bool over = tn == stop;  // both: f's end is not behind g's
-          ++i;
-          if (i == end || over)
-          {
-            done(part, sum.end());
-            ++part;
-            if (over || --parts == 0) break;
-            end += P.per;
-          }
-          f.advance();
+          done(sum.end());
+          if (tn == stop || --parts == 0) break;
+          k = 0;
         }
-        else g.advance();
+        if (first) f.advance(); else g.advance();
       }
     }
 
@@ -834,13 +823,13 @@ namespace sbg
     __device__ __noinline__ double walk_again(unsigned redo, const double* f, uint32_t nf, const double* g, uint32_t ng,
                                               uint64_t end, int scale, double res)
     {
-      const uint32_t lane = threadIdx.x & 31;
+      const uint32_t lane = threadIdx.x & 31, steps = 2 * nf;
+      // the end's time, rounded up
       const double stop = end == ~0ull ? tmax_of<double>() : ((double)end + 1.0) * pow2(-scale) * (1.0 + 0x1p-50);
-      DirectPair P;
-      if (__popc(redo) > MANY)
+      if (__popc(redo) * (12 + steps / 16) > steps)
       {
         if (!(redo >> lane & 1)) return res;
-        P.set<K, false>(f, nf, g, ng, stop);
+        const DirectPair P(f, nf, g, ng, stop, std::integral_constant<int, K>());
         // sums of 2^l neighbours that wait for the next 2^l, as the lanes add
         // them below; parts that are not there are zeros
         double wait[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -857,7 +846,7 @@ namespace sbg
           if (carry) res = s;
           ++n;
         };
-        direct_parts<K>(P, 0, 32, [&](uint32_t, double s) { push(s); });
+        direct_parts<K>(P, 0, 32, push);
         while (n < 32) push(0.0);
         return res;
       }
@@ -865,10 +854,10 @@ namespace sbg
       {
         const int k = __ffs((int)redo) - 1;
         redo &= redo - 1;
-        P.set<K, true>(f, nf, (const double*)__shfl_sync(FULL, (unsigned long long)g, k), __shfl_sync(FULL, ng, k),
-                       __shfl_sync(FULL, stop, k));
+        const DirectPair P(f, nf, (const double*)__shfl_sync(FULL, (unsigned long long)g, k), __shfl_sync(FULL, ng, k),
+                           __shfl_sync(FULL, stop, k), std::integral_constant<int, K>());
         double x = 0.0;
-        direct_parts<K>(P, lane, 1, [&](uint32_t, double s) { x = s; });
+        direct_parts<K>(P, lane, 1, [&](double s) { x = s; });
         __syncwarp();
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) x += __shfl_xor_sync(FULL, x, o);
@@ -959,7 +948,6 @@ namespace sbg
         const uint64_t* ctime = P.c.times + coff;
         const V* cval = cvals + coff;
         const double clast = P.c.pts[2 * (coff + cpoints) - 1];
-        const Shape cshape = P.c.shapes[corig];
 
         if (nrows > 0 && nrows <= P.rows_per_item)
         {
@@ -1104,17 +1092,21 @@ namespace sbg
                 const double tail = op_f64<K>(rlast, clast);
                 if (tail != 0.0) res = fma(tail, tmax_of<double>(), res);
               }
-              const uint64_t Tr = rlen > 1 ? A::units(rtime[rlen - 2]) : 0, Tc = clen > 1 ? A::units(ctime[clen - 2]) : 0;
-              const Shape rshape = P.r.shapes[iorig];
-              const unsigned redo = __ballot_sync(FULL, ok && !acc.good(rshape, cshape, Tr > Tc ? Tr : Tc));
-              if (redo)
-              {
-                // the products' end, where a side's last value is 0: its last
-                // change, rounded up
+              // the time of the later last change; products end where a side
+              // whose last value is 0 changes last (else ~0)
+              const auto last_change = [&](bool products) {
+                const uint64_t Tr = rlen > 1 ? A::units(rtime[rlen - 2]) : 0, Tc = clen > 1 ? A::units(ctime[clen - 2]) : 0;
                 uint64_t end = ~0ull;
                 if (K == OPK_INNER && rlast == 0.0) end = Tr;
                 if (K == OPK_INNER && clast == 0.0) end = Tc < end ? Tc : end;
-                res = walk_again<K>(redo, rpts, rpoints, P.c.pts + 2 * coff, cpoints, end, form.s, res);
+                return products || end != ~0ull ? end : Tr > Tc ? Tr : Tc;
+              };
+              const Shape rshape = P.r.shapes[iorig], cshape = P.c.shapes[corig];
+              const unsigned redo =
+                  __ballot_sync(FULL, ok && !acc.good(rshape, cshape, A::DROPS ? last_change(false) : 0));
+              if (redo)
+              {
+                res = walk_again<K>(redo, rpts, rpoints, P.c.pts + 2 * coff, cpoints, last_change(true), form.s, res);
                 __syncwarp();
               }
               if (ok)

@@ -27,9 +27,10 @@ namespace sbg
   };
 
   // What rounding can move of a PCF: the sum of |changes| at times that are no
-  // whole number of units, the largest |value| (both in integer values, general
-  // form: over 2^32), and for how long, in units, its value is no whole number.
-  struct alignas(16) Shape { float tv, vmax, ev, pad; };
+  // whole number of units, the largest |value|, for how long, in units, its value
+  // is no whole number, and the root of the sum of those changes' squares (values
+  // and changes as integer values, general form: over 2^32).
+  struct alignas(16) Shape { float tv, vmax, ev, rv; };
 
   // One side's PCFs: CSR, processing order, and the packed arrays of `cap`
   // elements (times, then values).
