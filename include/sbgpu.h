@@ -103,7 +103,11 @@ int sbg_get_device_verbose(void);
  * (1 caller's, 2 sorted
  * by breakpoint count), output bytes per pipeline band (automatic: 1/8 of
  * the output, the last eighth cut into halving parts so that little of the
- * copy-out runs after the last kernel). */
+ * copy-out runs after the last kernel).  The automatic choice for SBG_F64 L1,
+ * L2 and the L2 kernel is the fixed-point kernel, which takes at most 16 warps
+ * and 1024 rows per item (more are cut to those); a variant or a window cap
+ * selects one of the kernels above, which also run where the data does not suit
+ * fixed point. */
 int sbg_set_tuning(int warps, int row_chunk, int variant, int order, uint64_t band_bytes);
 
 /* Time-windowed variant: the most elements of one PCF inside a window
@@ -115,7 +119,8 @@ int sbg_get_window_cap(void);
 
 /* How host-buffer entry points return results: 0 automatic (= 1), 1 device
  * bands copied out through pinned staging buffers while the next band
- * computes, 2 the kernel stores straight into the caller's host buffer
+ * computes (a result of one band goes straight into the caller's pages where
+ * the device walks the host page tables), 2 the kernel stores straight into the caller's host buffer
  * (only on devices that use the host page tables, e.g. Grace + NVLink-C2C;
  * SBG_ERR_INVALID_ARGUMENT elsewhere). */
 int sbg_set_output_mode(int mode);
@@ -182,7 +187,11 @@ int sbg_pairwise_host(int dtype, int op, double p, int skip_mode,
  * breakpoint count over rows and columns (0: measured on the device, which
  * synchronises the stream).  row_perm / col_perm (optional, uint32) give the
  * processing order; results always land at the callers' (i, j).  Inputs are
- * not validated; malformed times cannot make the kernel read out of bounds. */
+ * not validated; malformed times cannot make the kernel read out of bounds.
+ * Scratch is stream-ordered and given back when the call's work is done.
+ * SBG_F64 L1, L2 and L2 kernel calls take 16 bytes per breakpoint (short PCFs,
+ * where nothing is read back: 16 * max_points bytes per PCF), and where that
+ * allocation fails run in double precision without it. */
 int sbg_pairwise_device(int dtype, int op, double p, int skip_mode,
                         const void* row_points, const uint64_t* row_offsets, uint64_t n_rows,
                         const void* col_points, const uint64_t* col_offsets, uint64_t n_cols,
@@ -279,7 +288,10 @@ void sbg_batch_destroy(sbg_batch* batch);
  * For callers that cannot allocate device memory when they need a matrix: an
  * application whose allocator owns all device memory, a component running
  * while a CUDA graph is being recorded around it, a plugin host that only lends
- * inputs and outputs.  Same computation and arguments as sbg_pairwise_device,
+ * inputs and outputs.  Same results, to rounding, and arguments as
+ * sbg_pairwise_device (SBG_F64 L1, L2 and L2 kernel calls run in double
+ * precision here, not in fixed point, whose packed arrays are larger than the
+ * scratch; their last bits differ),
  * plus the total breakpoint counts of the row and column sets; it calls no
  * cudaMalloc, cudaFree or other allocating routine.  Its scratch (the
  * persistent kernel's work-queue counter and, for PCFs too long for the
@@ -316,7 +328,8 @@ int sbg_pairwise_device_noalloc(int dtype, int op, double p, int skip_mode,
  *
  * sbg_autotune_device runs the problem (same arguments as
  * sbg_pairwise_device over the whole problem, results into out) for a few
- * (warps per CTA, rows per work item) shapes, times each with CUDA events on
+ * (warps per CTA, rows per work item) shapes (of the fixed-point kernel, where
+ * SBG_F64 calls take it), times each with CUDA events on
  * the stream (it synchronises), and caches the fastest under the problem's
  * key: element type, operation, skip mode and its shape bucket (floor(log2)
  * of n_rows and of max_points).  Later sbg_pairwise_device /

@@ -492,9 +492,15 @@ namespace
     ls.lmax = max_points; ls.lmin = 1; ls.mean = max_points;
     const Plan base = sbg::make_plan<T>(skip_mode, r.n, nc, ls, ls, dev, -1);
     std::vector<std::pair<int, int>> cands;
-    for (int w : {16, 24, 32})
-      for (uint32_t q : {base.q / 4, base.q / 2, base.q, base.q * 2})
-        if (q >= 1 && q <= 32) cands.push_back({w, (int)q});
+    if (sizeof(T) == 8 && takes_fixed_point(opk))  // at most 16 warps, whatever the direct kernel's plan
+    {
+      for (int w : {8, 12, 16})
+        for (int q : {1, 2, 4, 8}) cands.push_back({w, q});
+    }
+    else
+      for (int w : {16, 24, 32})
+        for (uint32_t q : {base.q / 4, base.q / 2, base.q, base.q * 2})
+          if (q >= 1 && q <= 32) cands.push_back({w, (int)q});
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     SBG_CUDA(cudaEventCreate(&e0));
     SBG_CUDA(cudaEventCreate(&e1));

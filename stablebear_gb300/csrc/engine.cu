@@ -771,6 +771,12 @@ namespace sbg
 
   // ---- double precision in fixed point (fixed_point.cu) ---------------------------
 
+  bool takes_fixed_point(int opk)
+  {
+    if (settings().variant.load() != 0 || settings().windowCap.load() != 0) return false;
+    return opk == OPK_L1 || opk == OPK_L2DIST || opk == OPK_INNER;
+  }
+
   namespace
   {
     // One call's fixed-point run: the record of its data, the packed arrays
@@ -778,7 +784,7 @@ namespace sbg
     // is launched behind every fixed one, gated by the record.
     struct FixedRun
     {
-      int opk = 0, sms = 0;
+      int opk = 0, sms = 0, warps = FIXED_WARPS;
       uint32_t q = 1, smem = 0, longest = 0;
       uint64_t rcap = 0, ccap = 0;
       bool cross = false;
@@ -804,11 +810,7 @@ namespace sbg
       // size (30 PCFs of L ~ U{16..200}, L1 on the device: 116 us a call
       // against 304 with the direct kernel, whose chain of FP64 latencies
       // alone is longer than all the launches here).
-      static bool wanted(int opk)
-      {
-        if (settings().variant.load() != 0 || settings().windowCap.load() != 0) return false;
-        return opk == OPK_L1 || opk == OPK_L2DIST || opk == OPK_INNER;
-      }
+      static bool wanted(int opk) { return takes_fixed_point(opk); }
       void layout(int opk_, int mode, uint64_t nr, uint64_t nc, uint32_t lmax, uint64_t row_points, uint64_t col_points,
                   uint64_t row_begin, const DeviceInfo& dev, int slots)
       {
@@ -818,13 +820,22 @@ namespace sbg
         cross = mode == MODE_CROSS;
         rcap = std::max<uint64_t>(row_points, 1);
         ccap = cross ? std::max<uint64_t>(col_points, 1) : rcap;
-        q = 1;
-        for (uint32_t cand : {4u, 2u})
-          if (row_begin % (32 * cand) == 0 && items_for(mode, 0, nr, nc, cand) >= (uint64_t)dev.sms * 6)
-          {
-            q = cand;
-            break;
-          }
+        // The launch shape the caller fixed, or the one measured for problems
+        // of this shape bucket; no sum depends on it.
+        int w = settings().warps.load(), chunk = settings().rowChunk.load();
+        if (w == 0 && chunk == 0) tune_cache_get(tune_key(8, opk, mode, nr, lmax), &w, &chunk);
+        if (w > 0) warps = std::min(w, FIXED_WARPS);
+        q = (uint32_t)std::min(chunk, 32);
+        if (q == 0)
+        {
+          q = 1;
+          for (uint32_t cand : {4u, 2u})
+            if (row_begin % (32 * cand) == 0 && items_for(mode, 0, nr, nc, cand) >= (uint64_t)dev.sms * 6)
+            {
+              q = cand;
+              break;
+            }
+        }
         smem = (uint32_t)(dev.smem_optin - 2048);
         auto up = [](size_t x) { return (x + 255) / 256 * 256; };
         rpack = 256;
@@ -838,7 +849,7 @@ namespace sbg
         // no sums pass from one to the next (a longer PCF than lmax does not
         // get there, by the record)
         const uint32_t slots_bytes = (32 * q * 4 + 15) / 16 * 16;
-        const bool one = lmax <= fixed_slice_cap(smem - slots_bytes, FIXED_WARPS, 16);
+        const bool one = lmax <= fixed_slice_cap(smem - slots_bytes, (uint32_t)warps, 16);
         carry_bytes = one ? 0 : up((size_t)sms * 32 * q * FIXED_CARRY * 32 * 8);
         total = carry + slots * carry_bytes;
       }
@@ -881,7 +892,7 @@ namespace sbg
         P.queue = queue(slot);
         if (used[slot]) SBG_CUDA(cudaMemsetAsync(P.queue, 0, 2 * sizeof(unsigned long long), st));
         used[slot] = true;
-        SBG_CUDA(launch_fixed_pairs(P, opk, (int)std::min<uint64_t>(P.n_items, (uint64_t)sms), st));
+        SBG_CUDA(launch_fixed_pairs(P, opk, warps, (int)std::min<uint64_t>(P.n_items, (uint64_t)sms), st));
         if (pl.packed)
         {
           d.rpts = static_cast<const double*>(rows());

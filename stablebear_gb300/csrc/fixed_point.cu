@@ -1183,7 +1183,7 @@ namespace sbg
     return launched();
   }
 
-  cudaError_t launch_fixed_pairs(const FixedParams& P, int opk, int grid, cudaStream_t st)
+  cudaError_t launch_fixed_pairs(const FixedParams& P, int opk, int warps, int grid, cudaStream_t st)
   {
     void (*fn)(const FixedParams) = opk == OPK_L1       ? fixed_pairs_kernel<OPK_L1>
                                     : opk == OPK_L2DIST ? fixed_pairs_kernel<OPK_L2DIST>
@@ -1192,7 +1192,7 @@ namespace sbg
     if (!fn) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.smem_bytes);
     if (e != cudaSuccess) return e;
-    fn<<<grid, FIXED_WARPS * 32, P.smem_bytes, st>>>(P);
+    fn<<<grid, warps * 32, P.smem_bytes, st>>>(P);
     return launched();
   }
 }

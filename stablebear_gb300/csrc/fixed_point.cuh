@@ -5,7 +5,7 @@
 
 namespace sbg
 {
-  // Warps per CTA, one CTA per SM.  Four warps a scheduler cover the walk's
+  // Warps per CTA unless the caller asks for fewer, one CTA per SM.  Four warps a scheduler cover the walk's
   // latencies, and 128 registers a thread hold it without spills (L1, general
   // values, N = 2500: 1.65 ms with 12 warps, 1.49 with 16, 1.57 with 20, 1.62
   // with 24).
@@ -75,5 +75,5 @@ namespace sbg
   cudaError_t launch_fixed_pack(const double* pts, const uint64_t* off, uint64_t n, uint64_t cap,
                                 FixedRecord* rec, int opk, void* packed, Shape* shapes, uint32_t* lens,
                                 bool elements, unsigned* gate, int sms, cudaStream_t st);
-  cudaError_t launch_fixed_pairs(const FixedParams& P, int opk, int grid, cudaStream_t st);
+  cudaError_t launch_fixed_pairs(const FixedParams& P, int opk, int warps, int grid, cudaStream_t st);
 }

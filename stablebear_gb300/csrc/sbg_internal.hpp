@@ -156,6 +156,10 @@ namespace sbg
     double mean = 0.0;
   };
 
+  // Whether automatic double calls of this operation take the fixed-point
+  // kernel (fixed_point.cu) under the present settings.
+  bool takes_fixed_point(int opk);
+
   // The float32 measurement variants 7 (replicated row, one unified load per
   // step) and 8 (merge path, one pair per warp), pair_variants.cu.
   cudaError_t launch_pair_variant(const LaunchParams<float>& L, int opk, int variant, int warps, int grid,

@@ -265,3 +265,46 @@ def test_small_values_are_as_exact_as_in_double_precision():
     X = sb.PcfArray.from_csr(*_join(lists))
     for which, j, want in (("l1", 40, 32 * v), ("l2", 40, np.sqrt(32.0) * v), ("kernel", 41, 24 * v)):
         assert abs(_pairs(X, which)(42, j) - want) <= 2.0 ** -51 * want, which
+
+
+def test_launch_shapes_are_the_callers():
+    """Warps and rows per item, set or cached, reach the float64 kernel: one
+    warp a CTA is far slower, and no shape changes a bit."""
+    import torch
+    import stablebear_gb300 as sb
+    from stablebear_gb300 import _native as nat
+    pts, off = _pcfs(np.random.default_rng(5).integers(20, 600, 900), "normal", seed=5)
+    n, longest = len(off) - 1, int(np.diff(off.astype(np.int64)).max())
+    dp, do = torch.from_numpy(pts).cuda(), torch.from_numpy(off.astype(np.int64)).cuda()
+    out = torch.empty(n * (n - 1) // 2, dtype=torch.float64, device="cuda")
+
+    def run():
+        best = float("inf")
+        for _ in range(4):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            nat.check(nat.lib().sbg_pairwise_device(nat.F64, nat.OP_L1, 1.0, nat.SKIP_LOWER_NODIAG, dp.data_ptr(),
+                                                    do.data_ptr(), n, None, None, 0, None, None, longest,
+                                                    out.data_ptr(), 0, 0, 0,
+                                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best, out.cpu().numpy().copy()
+
+    default, want = run()
+    try:
+        for warps, chunk in ((1, 0), (5, 1), (16, 8), (32, 32), (0, 3), (0, 1024)):
+            sb.set_tuning(warps=warps, row_chunk=chunk)
+            ms, got = run()
+            np.testing.assert_array_equal(got, want)
+            if warps == 1:
+                assert ms > 3 * default
+        sb.set_tuning()
+        nat.check(nat.lib().sbg_tuning_cache_store(nat.F64, nat.OP_L1, 1.0, nat.SKIP_LOWER_NODIAG, n, longest, 1, 64))
+        ms, got = run()
+        np.testing.assert_array_equal(got, want)
+        assert ms > 3 * default
+    finally:
+        sb.set_tuning()
+        nat.check(nat.lib().sbg_tuning_cache_clear())
