@@ -14,6 +14,8 @@
 #include "host_copy.hpp"
 #include "fixed_point.cuh"
 
+#include <cuda.h>  // CUcontext / CUresult types; the two driver calls are looked up through the runtime
+
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -82,25 +84,58 @@ namespace sbg
     }
   }
 
+  unsigned long long current_context_id()
+  {
+    using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+    using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
+    static CtxGetCurrentFn get_current = nullptr;
+    static CtxGetIdFn get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+      cudaDriverEntryPointQueryResult q;
+      void* fn = nullptr;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+          q == cudaDriverEntryPointSuccess)
+        get_current = reinterpret_cast<CtxGetCurrentFn>(fn);
+      fn = nullptr;
+      if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+          q == cudaDriverEntryPointSuccess)
+        get_id = reinterpret_cast<CtxGetIdFn>(fn);
+      cudaGetLastError();
+    });
+    if (!get_current || !get_id) throw Error(ST_CUDA, "cuCtxGetCurrent / cuCtxGetId not available from the driver");
+    CUcontext ctx = nullptr;
+    if (get_current(&ctx) != CUDA_SUCCESS || !ctx) return 0;
+    unsigned long long id = 0;
+    if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
+    return id;
+  }
+
   // Stream-ordered allocations come from one memory pool per device that
   // keeps up to POOL_KEEP bytes between calls; what is free above that goes
   // back to the device at the next synchronisation, and all of it when an
   // allocation of the library fails.  (The device's default pool keeps
   // nothing: after a synchronisation the next call's first allocation maps
   // memory again, 88 to 150 us against 2; a cudaFree is 55.)  The pool and
-  // its ordering between streams and threads are CUDA's own.
+  // its ordering between streams and threads are CUDA's own.  It goes with the
+  // context it was made in: after a device reset the next call makes another.
   static constexpr uint64_t POOL_KEEP = 256ull << 20;
-  static constexpr int POOL_DEVICES = 64;
 
   static cudaMemPool_t device_pool()
   {
     static std::mutex mu;
-    static cudaMemPool_t pools[POOL_DEVICES] = {};
+    static std::map<std::pair<int, unsigned long long>, cudaMemPool_t> pools;  // by device and context
     int dev = 0;
     SBG_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= POOL_DEVICES) return nullptr;
+    unsigned long long ctx = current_context_id();
+    if (ctx == 0)  // none yet in this thread
+    {
+      SBG_CUDA(cudaSetDevice(dev));  // makes the device's own current
+      ctx = current_context_id();
+    }
     std::lock_guard<std::mutex> lock(mu);
-    if (!pools[dev])
+    cudaMemPool_t& kept = pools[{dev, ctx}];
+    if (!kept)
     {
       cudaMemPoolProps props{};
       props.allocType = cudaMemAllocationTypePinned;
@@ -114,9 +149,9 @@ namespace sbg
       }
       uint64_t keep = POOL_KEEP;
       cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-      pools[dev] = pool;
+      kept = pool;
     }
-    return pools[dev];
+    return kept;
   }
 
   static cudaError_t pool_malloc(void** p, size_t bytes, cudaStream_t st)

@@ -13,8 +13,6 @@
 #include "../../include/sbgpu.h"
 #include "sbg_internal.hpp"
 
-#include <cuda.h>  // CUcontext / CUresult types; the two driver calls are looked up through the runtime
-
 #include <mutex>
 
 namespace sbg
@@ -35,37 +33,6 @@ namespace sbg
       unsigned long long context = 0;  // id of the CUDA context the address belongs to
     };
     ScratchAddr g_scratch_addr[kMaxDevices];
-
-    using CtxGetCurrentFn = CUresult (*)(CUcontext*);
-    using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
-
-    // Unique id of the calling thread's current CUDA context (cuCtxGetId), 0
-    // when none is current yet.  A device reset makes a new context with a
-    // new id, and the library module (with the array) is loaded anew in it.
-    unsigned long long current_context_id()
-    {
-      static CtxGetCurrentFn get_current = nullptr;
-      static CtxGetIdFn get_id = nullptr;
-      static std::once_flag once;
-      std::call_once(once, [] {
-        cudaDriverEntryPointQueryResult q;
-        void* fn = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-          get_current = reinterpret_cast<CtxGetCurrentFn>(fn);
-        fn = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &fn, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-          get_id = reinterpret_cast<CtxGetIdFn>(fn);
-        cudaGetLastError();
-      });
-      if (!get_current || !get_id) throw Error(ST_CUDA, "cuCtxGetCurrent / cuCtxGetId not available from the driver");
-      CUcontext ctx = nullptr;
-      if (get_current(&ctx) != CUDA_SUCCESS || !ctx) return 0;
-      unsigned long long id = 0;
-      if (get_id(ctx, &id) != CUDA_SUCCESS) return 0;
-      return id;
-    }
 
     // Device address of g_noalloc_scratch in the current device's context.
     // Host code only has a stand-in for the array, so the address is looked

@@ -110,6 +110,11 @@ namespace sbg
   };
   DeviceInfo device_info();
 
+  // Unique id of the calling thread's current CUDA context (cuCtxGetId), 0
+  // when none is current yet.  A device reset makes a new context with a
+  // new id, and the library module (with the array) is loaded anew in it.
+  unsigned long long current_context_id();
+
   // Resident CTAs per SM of a persistent pair kernel (64 registers per
   // thread, launch_bounds(1024, 1)) with `warps` warps and `smem_bytes` of
   // dynamic shared memory (plus 1 KB the runtime reserves per CTA).
