@@ -15,12 +15,19 @@
 //     (n x 2 bins), in FP32 FMAs;
 //   * inside a bin, at a breakpoint t_k of i, H_i adds w_ij times the steps of
 //     the other PCFs between the edge and t_k: a list of the bin's breakpoints
-//     against the breakpoints of i that lie there.
+//     against the breakpoints of i that lie there.  Its integral is taken over
+//     a segment's own part of the bin, not as a difference of two from the
+//     edge, which would keep the rounding of the whole bin in a segment of a
+//     thousandth of it; and in the last bin from its end, where H is that of
+//     zeros, since little is left there of what the edge's value sums.
 // Work per PCF pair falls from the merge's 2 L steps, with an atomic each, to
 // 2 bins FMAs and L^2 / bins list entries.  Nothing is added atomically, and
 // the sums are shorter.  N = 4096, L ~ U{16..512}, L2 kernel, forward and
 // backward: 14.4 -> 4.8 ms (the forward is 2.4 of it), error of the gradient
-// 8.5e-7 -> 3.1e-7.
+// 8.5e-7 -> 3.1e-7; of each value's gradient against the sum of its own
+// |terms|, N = 1000, segments from a millionth of a time unit on: rms 1.2e-8 to
+// 1.4e-8 over the first three quarters of the time and 3e-8 to 1.4e-7 behind,
+// 2.1e-8 in the walk (2.0 at the worst with differences from the edge).
 //
 // For distances each bin's mean value over the PCFs is taken off first: only
 // differences count there, and sums of w_ij g_j then stay as small as them.
@@ -509,11 +516,14 @@ namespace sbg
     // One CTA per group of up to 32 rows, whose weights lie in shared memory.
     // A warp takes a bin and the rows' breakpoints in it (lane r: row r), two
     // at a time: the bin's list up to a breakpoint's own place, weight times
-    // step (H), weight times step times distance (its integral).  Then each
-    // element's gradient from its two ends and the whole bins between.
+    // step (H), weight times step times distance, at most the element's part of
+    // the bin (its integral there).  Behind a row's last breakpoint of a bin lies
+    // what its elements leave of the whole bin's integral, or, of a quarter or
+    // less, the rest of the list.  Then each element's gradient from its parts
+    // and the whole bins between.
     // Bound by the list reads from L2 (the weights leave L1 no room for the
     // lists) and the gathers from shared memory: 1.2 ms at N = 4096, L ~
-    // U{16..512}, 608 bins.  Two breakpoints share a read; four waste as much
+    // U{16..512}, 576 bins.  Two breakpoints share a read; four waste as much
     // on the shorter prefixes (5.00 against 5.08 ms forward and backward),
     // one reads 14 GB (1.17 ms at 896 bins, L2 at 12 TB/s).  Unsorted lists
     // with a compare per entry took 1.75 ms at 896 bins.
@@ -570,13 +580,13 @@ namespace sbg
       // which the walk leaves out.
       bool lost = false;
 
-      // One breakpoint, from its bin's sums: H there, its time gradient, and
-      // the integral of H from the bin's edge to it.
-      auto finish = [&](uint32_t b, uint32_t e0, uint32_t e1, float edge, uint32_t r, uint32_t k, uint32_t at, float t,
+      // One breakpoint, from H at the bin's edge and its bin's sums: H there,
+      // its time gradient, and the integral of H over the last `width` before
+      // it (area: the part of the bin's list).  Returns that integral.
+      auto finish = [&](uint32_t b, uint32_t e0, uint32_t e1, float h0, float width, uint32_t r, uint32_t k, uint32_t at, float t,
                         float h, float area) {
         const uint64_t i = s_row[r], o = P.off[i];
         const float* w = smem + (size_t)r * n;
-        const float h0 = P.product[(i - P.r0) * 2 * P.bins + b];
         const float centre = KERNEL ? 0.0f : P.centre[b];
         float H = h0 + h, sum = KERNEL ? 0.0f : s_sum[r];
         if ((at > e0 && P.lists.event[at - 1].x == t) || (at + 1 < e1 && P.lists.event[at + 1].x == t))
@@ -620,9 +630,43 @@ namespace sbg
           float dt = KERNEL ? (a - c) * H : (a - c) * ((0.5f * ((a - centre) + (c - centre))) * sum - H);
           if (KERNEL) dt = fmaf(P.grad_out[i * (i + 1) / 2 + i], (a - c) * (a + c), dt);
           P.grad[2 * (o + k)] = dt;
-          P.area[o + k] = fmaf(h0, t - edge, area);
+          P.area[o + k] = fmaf(h0, width, area);
           lost |= !isfinite(dt);
         }
+        return fmaf(h0, width, area);
+      };
+      // A row's last breakpoint of a bin (its h as above): the integral of H
+      // from it to the bin's end.  What is left of the whole bin's, or, where
+      // that is less than a quarter and would keep the rounding of all of it,
+      // the entries from the breakpoint on.
+      auto finish_bin = [&](uint32_t b, uint32_t e1, float edge, float hi, uint32_t r, uint32_t k, uint32_t at, float t,
+                            float h, float before) {
+        const uint64_t i = s_row[r];
+        const float* product = P.product + (i - P.r0) * 2 * P.bins;
+        float rest = product[P.bins + b] - before;
+        if (hi - t < 0.25f * (hi - edge))
+        {
+          const float* w = smem + (size_t)r * n;
+          rest = 0.0f;
+          for (uint32_t c0 = at + 1 + lane; c0 < e1 + lane; c0 += 32 * AHEAD)
+          {
+            float2 ev[AHEAD];
+            uint32_t j[AHEAD];
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+            {
+              ev[u] = P.lists.event[c0 + 32 * u];
+              j[u] = P.lists.pcf[c0 + 32 * u];
+            }
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u)
+              rest = fmaf(w[j[u]] * (c0 + 32 * u < e1 ? ev[u].y : 0.0f), hi - ev[u].x, rest);
+          }
+#pragma unroll
+          for (int d = 16; d > 0; d >>= 1) rest += __shfl_xor_sync(FULL, rest, d);
+          rest = fmaf(product[b] + h, hi - t, rest);
+        }
+        if (lane == 0) P.rest[P.off[i] + k] = rest;
       };
 
       // this lane's row
@@ -636,23 +680,23 @@ namespace sbg
         if (lane == 0) b = atomicAdd(&s_bin, 1u);
         b = __shfl_sync(FULL, b, 0);
         if (b >= P.bins) break;
+        b = P.bins - 1 - b;  // the last bin first: it is walked whole for every breakpoint
         const uint32_t e0 = P.starts[b], e1 = P.starts[b + 1];
         if (e0 == e1) continue;
         const float edge = P.edges[b];
         // the row's breakpoints of this bin: [k0, k1); the last bin takes its end too
         const uint32_t k0 = mlen ? first_from(mp, mlen, edge) : 0;
         uint32_t k1 = k0;
+        const float hi = P.edges[b + 1];
         if (b + 1 == P.bins) k1 = mlen ? mlen : 0;
         else
-        {
-          const float hi = P.edges[b + 1];
           while (k1 < mlen && mp[2 * (uint64_t)k1] < hi) ++k1;
-        }
         uint32_t next = k0;
+        float before = 0.0f;  // integral of H from the bin's edge to this lane's row's breakpoints so far
         for (;;)
         {
           // up to BATCH breakpoints, a row after another
-          float t[BATCH], h[BATCH], area[BATCH];
+          float t[BATCH], width[BATCH], h[BATCH], area[BATCH], rest[BATCH];
           uint32_t row[BATCH], el[BATCH], place[BATCH], furthest = 0;
           int count = 0;
 #pragma unroll
@@ -660,13 +704,14 @@ namespace sbg
           {
             const unsigned left = __ballot_sync(FULL, next < k1);
             row[q] = el[q] = place[q] = 0;
-            t[q] = h[q] = area[q] = 0.0f;
+            t[q] = width[q] = h[q] = area[q] = rest[q] = 0.0f;
             if (!left) continue;
             row[q] = (uint32_t)__ffs((int)left) - 1;
             el[q] = __shfl_sync(FULL, next, row[q]);
             const uint64_t pt = __shfl_sync(FULL, moff, row[q]) + el[q];
             if (lane == (int)row[q]) ++next;
             t[q] = P.pts[2 * pt];
+            width[q] = t[q] - fmaxf(P.pts[2 * pt - 2], edge);  // of the element that ends here, in this bin
             place[q] = P.lists.place[pt];
             furthest = max(furthest, place[q]);
             ++count;
@@ -676,7 +721,33 @@ namespace sbg
           const float* w[BATCH];
 #pragma unroll
           for (int q = 0; q < BATCH; ++q) w[q] = smem + (size_t)row[q] * n;
-          for (uint32_t c0 = e0 + lane; c0 < furthest + lane; c0 += 32 * AHEAD)
+          // The last bin, where PCF after PCF has ended: back from its end, where
+          // H is that of zeros, and nothing is left of what has gone.
+          if (b + 1 == P.bins)
+          {
+            for (uint32_t c0 = e0 + lane; c0 < e1 + lane; c0 += 32 * AHEAD)
+            {
+              float2 ev[AHEAD];
+              uint32_t j[AHEAD];
+#pragma unroll
+              for (int u = 0; u < AHEAD; ++u)
+              {
+                ev[u] = P.lists.event[c0 + 32 * u];  // behind the list: zeros
+                j[u] = P.lists.pcf[c0 + 32 * u];
+              }
+#pragma unroll
+              for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+                for (int q = 0; q < BATCH; ++q)
+                {
+                  const float x = w[q][j[u]] * ev[u].y;
+                  h[q] -= c0 + 32 * u >= place[q] ? x : 0.0f;
+                  area[q] = fmaf(-x, fminf(fmaxf(ev[u].x - (t[q] - width[q]), 0.0f), width[q]), area[q]);
+                  rest[q] = fmaf(-x, fmaxf(ev[u].x - t[q], 0.0f), rest[q]);
+                }
+            }
+          }
+          else for (uint32_t c0 = e0 + lane; c0 < furthest + lane; c0 += 32 * AHEAD)
           {
             float2 ev[AHEAD];
             uint32_t j[AHEAD];
@@ -694,7 +765,7 @@ namespace sbg
               {
                 const float x = w[q][j[u]] * (c0 + 32 * u < place[q] ? ev[u].y : 0.0f);
                 h[q] += x;
-                area[q] = fmaf(x, t[q] - ev[u].x, area[q]);
+                area[q] = fmaf(x, fminf(t[q] - ev[u].x, width[q]), area[q]);
               }
           }
 #pragma unroll
@@ -707,7 +778,20 @@ namespace sbg
               h[q] += __shfl_xor_sync(FULL, h[q], d);
               area[q] += __shfl_xor_sync(FULL, area[q], d);
             }
-            finish(b, e0, e1, edge, row[q], el[q], place[q], t[q], h[q], area[q]);
+            const uint64_t i = s_row[row[q]];
+            const bool tail = b + 1 == P.bins;
+            const float h0 = !tail ? P.product[(i - P.r0) * 2 * P.bins + b] : KERNEL ? 0.0f : -P.centre[b] * s_sum[row[q]];
+            const float part = finish(b, e0, e1, h0, width[q], row[q], el[q], place[q], t[q], h[q], area[q]);
+            if (lane == (int)row[q]) before += part;
+            if (__shfl_sync(FULL, k1, row[q]) != el[q] + 1) continue;
+            if (tail)
+            {
+#pragma unroll
+              for (int d = 16; d > 0; d >>= 1) rest[q] += __shfl_xor_sync(FULL, rest[q], d);
+              if (lane == 0) P.rest[P.off[i] + el[q]] = fmaf(h0, hi - t[q], rest[q]);
+            }
+            else
+              finish_bin(b, e1, edge, hi, row[q], el[q], place[q], t[q], h[q], __shfl_sync(FULL, before, row[q]));
           }
         }
       }
@@ -728,25 +812,23 @@ namespace sbg
           const bool last = k + 1 == len;
           const float t1 = last ? P.edges[P.bins] : P.pts[2 * (o + k + 1)];
           const uint32_t b1 = last ? P.bins - 1 : P.bin[o + k + 1];
-          const float from = k ? P.area[o + k] : 0.0f;
-          const float to = last ? hint[P.bins - 1] : P.area[o + k + 1];
-          // whole bins, then the parts of the first and the last one
+          // the part of the first bin, whole bins, the part of the last one
           float H = 0.0f, own = 0.0f;
           if (b0 == b1)
           {
-            H = to - from;
+            H = !last ? P.area[o + k + 1] : k ? P.rest[o + k] : hint[b0];
             if (!KERNEL) own = (v - P.centre[b0]) * (t1 - t0);
           }
           else
           {
-            H = hint[b0] - from;
+            H = k ? P.rest[o + k] : hint[b0];
             if (!KERNEL) own = (v - P.centre[b0]) * (P.edges[b0 + 1] - t0);
             for (uint32_t b = b0 + 1; b < b1; ++b)
             {
               H += hint[b];
               if (!KERNEL) own = fmaf(v - P.centre[b], P.edges[b + 1] - P.edges[b], own);
             }
-            H += to;
+            H += last ? hint[b1] : P.area[o + k + 1];
             if (!KERNEL) own = fmaf(v - P.centre[b1], t1 - P.edges[b1], own);
           }
           float dv = KERNEL ? H : fmaf(own, sum, -H);
@@ -764,8 +846,9 @@ namespace sbg
   }
 
   // Bins (a multiple of 64): the product's waves of 128 x 128 tiles, about 75
-  // cycles for each k, against L^2 / bins list entries per pair of PCFs at two
-  // cycles for 32 of them (N = 4096, L ~ U{16..512}: 608 bins, product 0.70 ms
+  // cycles for each k (1.9 waves at N = 4096; the only wave of N = 1021, 104
+  // tiles, takes 2.4 times that), against L^2 / bins list entries per pair of PCFs at two
+  // cycles for 32 of them (N = 4096, L ~ U{16..512}: 576 bins, product 0.69 ms
   // and lists 1.2; with 896, 1.04 and 0.9 or more), and the table's entries.
   static uint32_t choose_bins(uint64_t n, uint64_t npts, int sms)
   {
@@ -829,6 +912,7 @@ namespace sbg
     p.point = add(npts * 4);
     p.place = add(npts * 4);
     p.area = add(npts * 4);
+    p.rest = add(npts * 4);
     p.bin = add(npts * 2);
     p.table = add(p.k * 2 * p.bins * 4);
     p.wt = add(p.k * p.width * 4);
@@ -895,7 +979,7 @@ namespace sbg
       L2Gradient G{};
       G.rec = rec; G.pts = pts; G.off = off; G.order = order; G.n = n; G.r0 = r0; G.width = p.width; G.rows = p.rows; G.bins = bins;
       G.edges = f32(p.edges); G.starts = u32(p.starts); G.centre = f32(p.centre); G.lists = lists;
-      G.wt = f32(p.wt); G.product = f32(p.product); G.grad_out = grad_out; G.grad = grad; G.area = f32(p.area);
+      G.wt = f32(p.wt); G.product = f32(p.product); G.grad_out = grad_out; G.grad = grad; G.area = f32(p.area); G.rest = f32(p.rest);
       G.bin = u16(p.bin);
       const uint64_t span = std::min<uint64_t>(p.width, n - r0);
       near<<<(unsigned)((span + p.rows - 1) / p.rows), NEAR_THREADS, near_smem, st>>>(G);

@@ -39,7 +39,8 @@ namespace sbg
     const float* product;   // [i - r0][2 bins]: H at the edges, its integral over the bins
     const float* grad_out;
     float* grad;            // (npts, 2): [dL/dt, dL/dv]
-    float* area;            // integral of H from the bin's edge to the breakpoint
+    float* area;            // integral of H up to the breakpoint, from the one before it or the bin's edge
+    float* rest;            // of the last breakpoint in a bin: from it to the bin's end
     const uint16_t* bin;    // the breakpoint's bin
   };
 
@@ -50,7 +51,7 @@ namespace sbg
     uint64_t k = 0, width = 0;  // rows of the table; rows of the gradient at a time
     size_t bytes = 0;
     size_t record = 0, edges = 0, counts = 0, starts = 0, next = 0, centre = 0, norm = 0, keys = 0, event = 0, pcf = 0, owner = 0,
-           point = 0, place = 0, area = 0, bin = 0, table = 0, wt = 0, product = 0;
+           point = 0, place = 0, area = 0, rest = 0, bin = 0, table = 0, wt = 0, product = 0;
   };
 
   // ok: false where the walk of backward.cu is the better one.

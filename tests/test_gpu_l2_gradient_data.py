@@ -102,3 +102,48 @@ def test_a_pcf_that_overflows(kind, size):
     got = _run(pts, off, kind, w)[1]
     assert bool((got[a:b] == 0).all())
     _near(got, _run(pts.double(), off, kind, w.double())[1])
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n,lo,hi", [(1000, 100, 200), (700, 300, 500), (2047, 60, 90)])
+def test_each_value_gradient_against_its_own_terms(kind, n, lo, hi):
+    """Segments from a millionth to a few units of time, far shorter and far
+    longer than a bin.  An entry sums w_ij times the integral of |g_j|, and of
+    |v| for distances, over its own segment: at most 256 + n / 256 rounded terms
+    of the product, a bin's list over 32 lanes (under 64 each), 14 more; where a
+    quarter of a bin is left of the whole, four times that."""
+    import torch
+    pts, off = _data(n, lo, hi, seed=n + 1)
+    rng = np.random.default_rng(n)
+    t = pts[:, 0].double().cpu().numpy()
+    gaps = np.diff(t, append=0.0)
+    short = rng.random(len(gaps)) < 0.3
+    gaps[short] *= 10.0 ** rng.uniform(-6, 0, short.sum())
+    o = off.cpu().numpy()
+    for a, b in zip(o[:-1], o[1:]):
+        t[a:b] = np.r_[0.0, np.cumsum(gaps[a:b - 1])]
+        x = t[a:b].astype(np.float32)
+        while np.any(np.diff(x) <= 0):  # times ascend in float32 too
+            at = np.nonzero(np.diff(x) <= 0)[0] + 1
+            x[at] = np.nextafter(x[at - 1], np.float32(np.inf))
+        t[a:b] = x
+    pts[:, 0] = torch.from_numpy(t).cuda()
+    w = _weights(n, kind, 9)
+    out, got = _run(pts, off, kind, w)
+    dout, want = _run(pts.double(), off, kind, w.double())
+    ap = pts.double().abs()
+    i, j = torch.tril_indices(n, n, 0 if kind == "kernel" else -1, device="cuda")
+    a = torch.zeros(n, n, device="cuda", dtype=torch.float64)
+    a[i, j] = w.double().abs() if kind == "kernel" else (w.double() / dout).abs()
+    k, m = torch.tril_indices(n, n, 0, device="cuda")
+    scale = _run(ap, off, "kernel", a[k, m])[1][:, 1]
+    if kind == "l2":
+        total = (a + a.T).sum(1)
+        owner = torch.repeat_interleave(torch.arange(n, device="cuda"), off[1:] - off[:-1])
+        width = torch.zeros(len(pts), device="cuda", dtype=torch.float64)
+        width[:-1] = (ap[1:, 0] - ap[:-1, 0]).clamp(min=0)
+        scale = scale + total[owner] * ap[:, 1] * width
+    last = torch.zeros(len(pts), dtype=torch.bool, device="cuda")
+    last[off[1:] - 1] = True
+    err = ((got[:, 1].double() - want[:, 1]).abs() / scale)[~last]
+    assert float(err.max()) <= 4 * (256 + n / 256 + 64 + 14) * 2.0 ** -24, float(err.max())
