@@ -33,6 +33,7 @@
 
 #include "fixed_point.cuh"
 
+#include <cfloat>
 #include <type_traits>
 
 namespace sbg
@@ -117,7 +118,10 @@ namespace sbg
     // and op(f', g') - op(f, g) is at most
     //   L1        |f' - f| + |g' - g|
     //   products  |f' - f| max |g| + |g' - g| max |f|
-    //   squares   (|f' - f| + |g' - g|) 2 (max |f| + max |g|).
+    //   squares   (|f' - f| + |g' - g|) 2 max |f - g|.
+    // Times that round lie below 2^52 units, so their share has the maxima of
+    // what starts there, for squares that of the two ranges' distance: PCFs that
+    // start alike are as close there as they are large elsewhere.
     // (0.501 for a half: the floats here round.)  Roundings of times in both
     // directions even out: usually a third of the root of the sum of squares
     // stands for half the sum.  A pair is taken if its usual error is at most
@@ -134,28 +138,41 @@ namespace sbg
         return worst <= total * 0x1p-47f && usual <= total * (opk == OPK_L2DIST ? 0x1p-50f : 0x1p-51f);
       }
     };
-    __device__ __forceinline__ float moved(int opk, const Shape& f, const Shape& g, float df, float dg)
-    {
-      if (opk == OPK_L1) return 0.501f * (df + dg);
-      if (opk == OPK_INNER) return 0.501f * (df * g.vmax + dg * f.vmax);
-      return 1.002f * (df + dg) * (f.vmax + g.vmax);
-    }
+    // Times, in integer values (general: over 2^32, squares and products over 2^64).
     __device__ __forceinline__ Bound counts_bound(int opk, const Shape& f, const Shape& g)
     {
-      // (products of general values are beyond a float when squared)
-      const float a = opk == OPK_INNER ? f.rv * 0x1p-20f * (g.vmax * 0x1p-20f) : f.rv;
-      const float b = opk == OPK_INNER ? g.rv * 0x1p-20f * (f.vmax * 0x1p-20f) : g.rv;
-      const float scale = opk == OPK_L1 ? 1.0f : opk == OPK_INNER ? 0x1p40f : 2.0f * (f.vmax + g.vmax);
-      return Bound{moved(opk, f, g, f.tv, g.tv), 0.289f * sqrtf(fmaf(a, a, b * b)) * scale};
+      float worst, a = f.rv, b = g.rv, scale = 1.0f;
+      if (opk == OPK_INNER)
+      {
+        const float mf = fmaxf(fabsf(f.lo), fabsf(f.hi)), mg = fmaxf(fabsf(g.lo), fabsf(g.hi));
+        worst = 0.501f * (f.tv * mg + g.tv * mf);
+        a *= 0x1p-20f * (mg * 0x1p-20f);  // general products are beyond a float when squared
+        b *= 0x1p-20f * (mf * 0x1p-20f);
+        scale = 0x1p40f;
+      }
+      else if (opk == OPK_L2DIST)
+      {
+        // (the ranges' own rounding to floats included)
+        const float far = fmaxf(f.hi - g.lo, g.hi - f.lo) +
+                          0x1p-22f * (fabsf(f.lo) + fabsf(f.hi) + fabsf(g.lo) + fabsf(g.hi));
+        worst = 1.002f * (f.tv + g.tv) * far;
+        scale = 2.0f * far;
+      }
+      else worst = 0.501f * (f.tv + g.tv);
+      return Bound{worst, 0.289f * sqrtf(fmaf(a, a, b * b)) * scale};
     }
-    // Shapes' values are in units of 2^32 here, their times are not; products
-    // and squares are in units of 2^64 and drop up to one of those up to the
-    // time T from which they are 0.
+    // And values, whose times count over all of the PCF; products and squares
+    // drop up to one unit up to the time T from which they are 0.
     __device__ __forceinline__ Bound general_bound(int opk, const Shape& f, const Shape& g, float T)
     {
       const Bound t = counts_bound(opk, f, g);
-      const float v = moved(opk, f, g, f.ev, g.ev);
-      if (opk == OPK_L1) return Bound{fmaf(t.worst, 0x1p32f, v), fmaf(t.usual, 0x1p32f, v)};
+      if (opk == OPK_L1)
+      {
+        const float v = 0.501f * (f.ev + g.ev);
+        return Bound{fmaf(t.worst, 0x1p32f, v), fmaf(t.usual, 0x1p32f, v)};
+      }
+      const float v = opk == OPK_INNER ? 0.501f * (f.ev * g.vmax + g.ev * f.vmax)
+                                       : 1.002f * (f.ev + g.ev) * (f.vmax + g.vmax);
       return Bound{fmaf(v, 0x1p-32f, t.worst) + T, fmaf(v, 0x1p-32f, t.usual) + T};
     }
 
@@ -296,7 +313,7 @@ namespace sbg
           if (elements) write_elements(pts, o, len, static_cast<Elem<double>*>(packed), lane);
           continue;
         }
-        float tv = 0.0f, qv = 0.0f, ev = 0.0f, vm = 0.0f, area = 0.0f, end = 0.0f;
+        float tv = 0.0f, qv = 0.0f, ev = 0.0f, vm = 0.0f, area = 0.0f, end = 0.0f, lo = FLT_MAX, hi = -FLT_MAX;
         uint64_t count = 0;  // elements before this chunk
         for (uint64_t k0 = 0; k0 < len; k0 += 32)
         {
@@ -318,6 +335,7 @@ namespace sbg
           {
             const uint64_t at = o + count + __popc(mask & ((1u << lane) - 1u));  // <= o + k
             const long long F = __double2ll_rn(v * vs);
+            const float value = (float)F * (f.kind == 1 ? 1.0f : 0x1p-32f);
             if (k > 0)
             {
               if (!whole(t, f.s))
@@ -330,7 +348,12 @@ namespace sbg
               end = scaled(t, f.s);
               area = fmaf(opk == OPK_L1 ? fabsf(x) - fabsf(y) : (x - y) * (x + y), end, area);
             }
-            vm = fmaxf(vm, fabsf((float)F) * (f.kind == 1 ? 1.0f : 0x1p-32f));
+            if (k == 0 || end < 0x1p52f)  // (cut off, so right at the border)
+            {
+              lo = fminf(lo, value);
+              hi = fmaxf(hi, value);
+            }
+            vm = fmaxf(vm, fabsf(value));
             if (f.kind == 1)
               static_cast<uint32_t*>(values)[at] = (uint32_t)(int32_t)F;
             else
@@ -354,12 +377,14 @@ namespace sbg
           vm = fmaxf(vm, __shfl_xor_sync(FULL, vm, h));
           area += __shfl_xor_sync(FULL, area, h);
           end = fmaxf(end, __shfl_xor_sync(FULL, end, h));
+          lo = fminf(lo, __shfl_xor_sync(FULL, lo, h));
+          hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, h));
         }
         if (lane == 0)
         {
           times[o + count - 1] = f.kind == 1 ? ((T_END >> 31) << 32) | (T_END & 0x7fffffffull) : T_END;
           lens[i] = (uint32_t)count;
-          const Shape s{tv, vm, ev, sqrtf(qv)};
+          const Shape s{tv, sqrtf(qv), lo, hi, vm, ev, 0.0f, 0.0f};
           shapes[i] = s;
           // a pair with one like it: |f - g| is about |f|, its square twice that
           // of f, |f g| some five eighths of it

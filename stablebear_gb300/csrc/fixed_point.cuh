@@ -27,10 +27,11 @@ namespace sbg
   };
 
   // What rounding can move of a PCF: the sum of |changes| at times that are no
-  // whole number of units, the largest |value|, for how long, in units, its value
-  // is no whole number, and the root of the sum of those changes' squares (values
-  // and changes as integer values, general form: over 2^32).
-  struct alignas(16) Shape { float tv, vmax, ev, rv; };
+  // whole number of units, and the root of the sum of their squares; the range of
+  // its values where times may round, before 2^52 units; its largest |value|;
+  // and for how long, in units, its value is no whole number.  (Values and
+  // changes as integer values, general form: over 2^32.)
+  struct alignas(16) Shape { float tv, rv, lo, hi, vmax, ev, pad[2]; };
 
   // One side's PCFs: CSR, processing order, and the packed arrays of `cap`
   // elements (times, then values).
