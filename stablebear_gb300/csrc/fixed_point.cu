@@ -34,7 +34,6 @@
 #include "fixed_point.cuh"
 
 #include <cfloat>
-#include <type_traits>
 
 namespace sbg
 {
@@ -707,8 +706,8 @@ namespace sbg
     //
     // Only what comes before `stop` counts, at or after the time from which
     // every term is 0 (the largest double: no such time): the products of a
-    // PCF that ends early are over when it is, and the other's thousands of
-    // later elements add nothing (the L2 kernel of 3500 stable ranks with a few
+    // PCF that ends early are over when it is, the distances of two when both
+    // are, and thousands of later elements add nothing (the L2 kernel of 3500 stable ranks with a few
     // such: 2.98 ms with them, 0.98 without).
     __device__ __forceinline__ uint32_t elements_before(const double* f, uint32_t n, double stop)
     {
@@ -727,12 +726,11 @@ namespace sbg
       uint32_t nf, ng, per;  // elements; breakpoints of a part, the end at `stop` one of them
       double stop;           // where both sides' last elements end
 
-      template <int K>
       __device__ __forceinline__ DirectPair(const double* f_, uint32_t nf_, const double* g_, uint32_t ng_,
-                                            double stop_, std::integral_constant<int, K>)
+                                            double stop_)
           : f(f_), g(g_), nf(nf_), ng(ng_), stop(stop_)
       {
-        if (K == OPK_INNER && stop < tmax_of<double>())
+        if (stop < tmax_of<double>())
         {
           nf = elements_before(f, nf, stop);
           ng = elements_before(g, ng, stop);
@@ -854,7 +852,7 @@ namespace sbg
       if (__popc(redo) * (12 + steps / 16) > steps)
       {
         if (!(redo >> lane & 1)) return res;
-        const DirectPair P(f, nf, g, ng, stop, std::integral_constant<int, K>());
+        const DirectPair P(f, nf, g, ng, stop);
         // sums of 2^l neighbours that wait for the next 2^l, as the lanes add
         // them below; parts that are not there are zeros
         double wait[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -880,7 +878,7 @@ namespace sbg
         const int k = __ffs((int)redo) - 1;
         redo &= redo - 1;
         const DirectPair P(f, nf, (const double*)__shfl_sync(FULL, (unsigned long long)g, k), __shfl_sync(FULL, ng, k),
-                           __shfl_sync(FULL, stop, k), std::integral_constant<int, K>());
+                           __shfl_sync(FULL, stop, k));
         double x = 0.0;
         direct_parts<K>(P, lane, 1, [&](double s) { x = s; });
         __syncwarp();
@@ -1117,21 +1115,22 @@ namespace sbg
                 const double tail = op_f64<K>(rlast, clast);
                 if (tail != 0.0) res = fma(tail, tmax_of<double>(), res);
               }
-              // the time of the later last change; products end where a side
-              // whose last value is 0 changes last (else ~0)
-              const auto last_change = [&](bool products) {
+              // The time from which every term is 0: of products where a side
+              // whose last value is 0 changes last, of distances where the
+              // later side does, if the last values are alike; else `none`.
+              const auto end = [&](bool later_change) -> uint64_t {
                 const uint64_t Tr = rlen > 1 ? A::units(rtime[rlen - 2]) : 0, Tc = clen > 1 ? A::units(ctime[clen - 2]) : 0;
-                uint64_t end = ~0ull;
-                if (K == OPK_INNER && rlast == 0.0) end = Tr;
-                if (K == OPK_INNER && clast == 0.0) end = Tc < end ? Tc : end;
-                return products || end != ~0ull ? end : Tr > Tc ? Tr : Tc;
+                const uint64_t none = later_change ? (Tr > Tc ? Tr : Tc) : ~0ull;
+                if (K != OPK_INNER) return rlast == clast ? (Tr > Tc ? Tr : Tc) : none;
+                if (rlast == 0.0 && clast == 0.0) return Tr < Tc ? Tr : Tc;
+                return rlast == 0.0 ? Tr : clast == 0.0 ? Tc : none;
               };
               const Shape rshape = P.r.shapes[iorig], cshape = P.c.shapes[corig];
               const unsigned redo =
-                  __ballot_sync(FULL, ok && !acc.good(rshape, cshape, A::DROPS ? last_change(false) : 0));
+                  __ballot_sync(FULL, ok && !acc.good(rshape, cshape, A::DROPS ? end(true) : 0));
               if (redo)
               {
-                res = walk_again<K>(redo, rpts, rpoints, P.c.pts + 2 * coff, cpoints, last_change(true), form.s, res);
+                res = walk_again<K>(redo, rpts, rpoints, P.c.pts + 2 * coff, cpoints, end(false), form.s, res);
                 __syncwarp();
               }
               if (ok)
