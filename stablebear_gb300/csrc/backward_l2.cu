@@ -24,7 +24,7 @@
 // 2 bins FMAs and L^2 / bins list entries.  Nothing is added atomically, and
 // the sums are shorter.  N = 4096, L ~ U{16..512}, L2 kernel, forward and
 // backward: 14.4 -> 4.8 ms (the forward is 2.4 of it), error of the gradient
-// 8.5e-7 -> 3.1e-7; of each value's gradient against the sum of its own
+// 8.5e-7 -> 3.0e-7; of each value's gradient against the sum of its own
 // |terms|, N = 1000, segments from a millionth of a time unit on: rms 1.2e-8 to
 // 1.4e-8 over the first three quarters of the time and 3e-8 to 1.4e-7 behind,
 // 2.1e-8 in the walk (with differences from the edge up to 20, rms 5e-2).
@@ -522,7 +522,7 @@ namespace sbg
     // less, the rest of the list.  Then each element's gradient from its parts
     // and the whole bins between.
     // Bound by the list reads from L2 (the weights leave L1 no room for the
-    // lists) and the gathers from shared memory: 1.2 ms at N = 4096, L ~
+    // lists) and the gathers from shared memory: 1.4 ms at N = 4096, L ~
     // U{16..512}, 576 bins.  Two breakpoints share a read; four waste as much
     // on the shorter prefixes (5.00 against 5.08 ms forward and backward),
     // one reads 14 GB (1.17 ms at 896 bins, L2 at 12 TB/s).  Unsorted lists
