@@ -218,10 +218,14 @@ int sbg_measure_peak(int kind, double* lane_ops_per_s);
  * L1) or L2 kernel problem, writes dL/d(points) into grad_points, laid out
  * like the points: (n_points, 2) pairs [dL/dt, dL/dv].  forward_out is the
  * forward result M (needed for the L2 distance, optional otherwise).  The
- * merge is recomputed.  Times that coincide with a breakpoint of the other
- * PCF of a pair (ties) and each PCF's first time t = 0 get no gradient from
- * that pair.  Accumulation uses atomic adds (order not deterministic).
- * Device pointers, stream-ordered; grad_points is overwritten. */
+ * merge is recomputed; or, for SBG_F32 L2 distances and kernels of 300 and
+ * more PCFs, the gradient is a contraction over time bins, with scratch of
+ * 4 n^2 bytes (at most 1 GB) and tables, and the merge where that is refused.
+ * Times that coincide with a breakpoint of the other PCF of a pair (ties) and
+ * each PCF's first time t = 0 get no gradient from that pair.  The merge
+ * accumulates with atomic adds (order not deterministic), the contraction only
+ * for pairs of distances far smaller than their PCFs.  Points that no offsets
+ * cover get 0.  Device pointers, stream-ordered; grad_points is overwritten. */
 int sbg_pairwise_backward_device(int dtype, int op, double p, int skip_mode,
                                  const void* points, const uint64_t* offsets, uint64_t n, uint64_t n_points,
                                  uint32_t max_points, const void* grad_out, const void* forward_out,
