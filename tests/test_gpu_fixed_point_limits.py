@@ -308,3 +308,47 @@ def test_launch_shapes_are_the_callers():
     finally:
         sb.set_tuning()
         nat.check(nat.lib().sbg_tuning_cache_clear())
+
+
+@pytest.mark.parametrize("values", ["counts", "normal"])
+def test_one_last_value_that_is_not_zero(values):
+    """A single PCF that never returns to zero: its last rectangle reaches to
+    the largest double, as in the direct kernels."""
+    import stablebear_gb300 as sb
+    pts, off = _pcfs(np.random.default_rng(3).integers(1, 300, 70), values, seed=3)
+    pts[int(off[4]) - 1, 1] = 5.0
+    X = sb.PcfArray.from_csr(pts, off)
+
+    def every():
+        return [sb.pdist(X).data.copy(), sb.pdist(X, p=2).data.copy(), sb.l2_kernel(X).data.copy()]
+
+    got = every()
+    try:
+        sb.set_tuning(variant=5)
+        want = every()
+    finally:
+        sb.set_tuning()
+    for a, b in zip(got, want):
+        finite = np.isfinite(b)
+        np.testing.assert_array_equal(np.isfinite(a), finite)
+        np.testing.assert_array_equal(a[~finite], b[~finite])
+        big = finite & (np.abs(b) > 1e100)
+        np.testing.assert_allclose(a[big], b[big], rtol=TOL)
+
+
+@pytest.mark.parametrize("values", ["counts", "normal"])
+def test_equal_last_values_that_are_not_zero(values):
+    """Distances of PCFs that end on one value other than 0 end where the later
+    one does, also for pairs that are walked again."""
+    import stablebear_gb300 as sb
+    from oracle import oracle as orc
+    pts, off = _pcfs(np.random.default_rng(4).integers(1, 200, 60), values, seed=4)
+    pts[off[1:].astype(np.int64) - 1, 1] = 7.0
+    for i in range(0, 60, 3):  # early ones, with points behind their last change
+        a, b = int(off[i]), int(off[i + 1])
+        pts[a:b, 0] *= 1e-9
+        pts[a + (b - a) // 2:b, 1] = 7.0
+    X = sb.PcfArray.from_csr(pts, off)
+    for got, kw in ((sb.pdist(X).data, dict(op=orc.OP_L1)), (sb.pdist(X, p=2).data, dict(op=orc.OP_LP, p=2.0))):
+        want = orc.evaluate(pts, off, mode=orc.MODE_PDIST, truth=True, **kw)
+        assert np.all(np.abs(got - want) <= TOL * want)
