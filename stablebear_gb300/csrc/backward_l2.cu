@@ -34,8 +34,8 @@
 // Pairs that lie close together beside that are left to the walk (l2_close).
 //
 // A weight or a value that is not finite, a last value other than 0 (its
-// integral has no end), times that do not ascend or a gradient that comes out
-// not finite make the walk of backward.cu run instead, decided by a record on
+// integral has no end), times out of order or a gradient that comes out not
+// finite make the walk of backward.cu run instead, decided by a record on
 // the device.
 #include "sbg_internal.hpp"
 
@@ -56,13 +56,18 @@ namespace sbg
     constexpr int AHEAD = 4;            // list entries a lane has in flight
     constexpr uint32_t BIN_MAX = 8192;  // breakpoints of a bin
 
+    // A time >= 0 as bits that order like it (-0, which passes for 0 in every
+    // comparison of times, would order above them all).
+    __device__ __forceinline__ uint32_t time_bits(float t) { return t > 0.0f ? __float_as_uint(t) : 0u; }
+
     // Times from the second breakpoint on (the first is the start whatever it
-    // says) have to ascend from above 0: at an element without width the walk
-    // gives the pair's row a time gradient and its column none.  That also
-    // keeps out -0, whose bits order above every other time's.
+    // says) must not descend from 0.  The breakpoints behind elements without
+    // width are listed, for l2_narrow_kernel: up to n of them, more make the
+    // data the walk's.
     __global__ void __launch_bounds__(256) l2_record_kernel(const float* __restrict__ pts,
                                                             const uint64_t* __restrict__ off, uint64_t n,
-                                                            uint64_t npts, L2Record* rec)
+                                                            uint64_t npts, L2Record* rec,
+                                                            uint32_t* __restrict__ narrow)
     {
       const int lane = threadIdx.x & 31;
       const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -80,8 +85,14 @@ namespace sbg
           if (k > 0)
           {
             const float t = pts[2 * (o + k)], before = k > 1 ? pts[2 * (o + k - 1)] : 0.0f;
-            bad |= !(t > before) || !(t < FLT_MAX) ? 1u : 0u;
-            tmax = max(tmax, __float_as_uint(t));
+            bad |= !(t >= before) || !(t < FLT_MAX) ? 1u : 0u;
+            if (t == before)
+            {
+              const uint32_t at = atomicAdd(&rec->narrow, 1u);
+              if (at < n) narrow[at] = (uint32_t)(o + k);
+              else bad = 1;
+            }
+            tmax = max(tmax, time_bits(t));
           }
         }
       }
@@ -194,7 +205,7 @@ namespace sbg
         const uint64_t o = off[i], len = off[i + 1] - o;
         for (uint64_t k = 1 + lane; k < len; k += 32)
           keys[atomicAdd(&place[bin[o + k]], 1u)] =
-              ((uint64_t)__float_as_uint(pts[2 * (o + k)]) << 32) | (uint32_t)(o + k);
+              ((uint64_t)time_bits(pts[2 * (o + k)]) << 32) | (uint32_t)(o + k);
       }
     }
 
@@ -842,6 +853,68 @@ namespace sbg
       if (__any_sync(FULL, lost) && lane == 0) atomicOr(&P.rec->bad_weights, 1u);
     }
 
+    // Time gradients behind elements without width, which the walks give the
+    // row of a pair alone, the later PCF in length order: a column's step of
+    // width 0 passes for a tie.  One CTA per breakpoint, over the earlier PCFs.
+    template <bool KERNEL>
+    __global__ void __launch_bounds__(256) l2_narrow_kernel(const __grid_constant__ L2Gradient P)
+    {
+      __shared__ uint32_t s_closed, s_place;
+      __shared__ float s_part[8];
+      if (threadIdx.x == 0)
+      {
+        s_closed = P.rec->bad | P.rec->bad_weights;  // bad_weights may be set meanwhile
+        s_place = 0;
+      }
+      __syncthreads();
+      if (s_closed) return;
+      const uint32_t count = P.rec->narrow;
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      for (uint32_t x = blockIdx.x; x < count; x += gridDim.x)
+      {
+        const uint64_t pt = P.narrow[x], i = P.owner[pt];
+        const float t = P.pts[2 * pt], a = P.pts[2 * pt - 1], c = P.pts[2 * pt + 1];
+        // the PCF's place in length order, which stays within its window
+        const uint64_t w0 = i / LENGTH_ORDER_WINDOW * LENGTH_ORDER_WINDOW, w1 = min(w0 + LENGTH_ORDER_WINDOW, P.n);
+        for (uint64_t p = w0 + threadIdx.x; p < w1; p += 256)
+          if (P.order[p] == i) s_place = (uint32_t)p;
+        __syncthreads();
+        float sum = 0.0f;
+        for (uint32_t p = threadIdx.x; p < s_place; p += 256)
+        {
+          const uint64_t j = P.order[p], hi = max(i, j), lo = min(i, j);
+          const uint64_t at = KERNEL ? hi * (hi + 1) / 2 + lo : hi * (hi - 1) / 2 + lo;
+          float w = P.grad_out[at];
+          if (!KERNEL)
+          {
+            const float d = P.fwd[at];
+            w = d > 0.0f ? w / d : 0.0f;
+            if (w != 0.0f && l2_close(d, P.norm[hi], P.norm[lo])) w = 0.0f;
+          }
+          if (w == 0.0f) continue;
+          const uint64_t o = P.off[j];
+          const uint32_t len = (uint32_t)(P.off[j + 1] - o), k = first_from(P.pts + 2 * o, len, t);
+          if (k < len && P.pts[2 * (o + k)] == t) continue;  // a tie
+          const float g = P.pts[2 * (o + k) - 1];
+          sum = fmaf(w, KERNEL ? g : 0.5f * (a + c) - g, sum);
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(FULL, sum, d);
+        if (lane == 0) s_part[warp] = sum;
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+          float all = 0.0f;
+          for (int q = 0; q < 8; ++q) all += s_part[q];
+          float dt = (a - c) * all;
+          if (KERNEL) dt = fmaf(P.grad_out[i * (i + 1) / 2 + i], (a - c) * (a + c), dt);
+          P.grad[2 * pt] = dt;
+          if (!isfinite(dt)) atomicOr(&P.rec->bad_weights, 1u);
+        }
+        __syncthreads();
+      }
+    }
+
     uint64_t up(uint64_t x, uint64_t to) { return (x + to - 1) / to * to; }
   }
 
@@ -905,6 +978,7 @@ namespace sbg
     p.next = add(p.bins * 4);
     p.centre = add(p.bins * 4);
     p.norm = add(n * 4);
+    p.narrow = add(n * 4);
     p.keys = add(npts * 8);
     p.event = add((npts + 32 * AHEAD) * 8);  // the sums read past a list's end
     p.pcf = add((npts + 32 * AHEAD) * 2);
@@ -933,7 +1007,7 @@ namespace sbg
     const uint32_t bins = p.bins;
     const unsigned warps8 = (unsigned)std::min<uint64_t>((n + 7) / 8, (uint64_t)dev.sms * 8);
     SBG_CUDA(cudaMemsetAsync(base + p.record, 0, p.starts - p.record, st));  // the record and the counts
-    l2_record_kernel<<<warps8, 256, 0, st>>>(pts, off, n, npts, rec);
+    l2_record_kernel<<<warps8, 256, 0, st>>>(pts, off, n, npts, rec, u32(p.narrow));
     SBG_CUDA(launched());
     l2_edges_kernel<<<1, 1024, 0, st>>>(pts, off, n, rec, bins, f32(p.edges));
     SBG_CUDA(launched());
@@ -968,6 +1042,7 @@ namespace sbg
     const size_t near_smem = (size_t)p.rows * n * sizeof(float);
     void (*near)(const L2Gradient) = kernel ? l2_gradient_kernel<true> : l2_gradient_kernel<false>;
     SBG_CUDA(cudaFuncSetAttribute(near, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)near_smem));
+    L2Gradient G{};
     for (uint64_t r0 = 0; r0 < n; r0 += p.width)
     {
       const dim3 tiles((unsigned)(p.width / 32), (unsigned)((p.k + 31) / 32));
@@ -976,7 +1051,6 @@ namespace sbg
       l2_product_kernel<<<dim3(2 * bins / GT, (unsigned)(p.width / GT)), 256, gemm_smem, st>>>(
           f32(p.wt), p.width, f32(p.table), 2 * bins, p.k, rec, f32(p.product));
       SBG_CUDA(launched());
-      L2Gradient G{};
       G.rec = rec; G.pts = pts; G.off = off; G.order = order; G.n = n; G.r0 = r0; G.width = p.width; G.rows = p.rows; G.bins = bins;
       G.edges = f32(p.edges); G.starts = u32(p.starts); G.centre = f32(p.centre); G.lists = lists;
       G.wt = f32(p.wt); G.product = f32(p.product); G.grad_out = grad_out; G.grad = grad; G.area = f32(p.area); G.rest = f32(p.rest);
@@ -985,6 +1059,9 @@ namespace sbg
       near<<<(unsigned)((span + p.rows - 1) / p.rows), NEAR_THREADS, near_smem, st>>>(G);
       SBG_CUDA(launched());
     }
+    G.narrow = u32(p.narrow); G.owner = u16(p.owner); G.fwd = fwd; G.norm = f32(p.norm);
+    (kernel ? l2_narrow_kernel<true> : l2_narrow_kernel<false>)<<<(unsigned)std::min<uint64_t>(n, (uint64_t)dev.sms * 8), 256, 0, st>>>(G);
+    SBG_CUDA(launched());
     *norms = f32(p.norm);
     return &rec->bad;
   }

@@ -8,7 +8,8 @@ namespace sbg
   // What the data of a call is like, gathered on the device (zeroed first).
   // bad: the data takes the walk; bad_weights: a weight, an overfull bin or a
   // gradient that is not finite does; close: some pairs of distances do (l2_close).
-  struct L2Record { uint32_t bad, bad_weights, close, tmax_bits; };
+  // narrow: breakpoints behind elements without width.
+  struct L2Record { uint32_t bad, bad_weights, close, tmax_bits, narrow; };
 
   // A distance far smaller than its two PCFs (less the common part): in
   // v S - H its weight w / D would multiply their size, not their difference,
@@ -42,6 +43,10 @@ namespace sbg
     float* area;            // integral of H up to the breakpoint, from the one before it or the bin's edge
     float* rest;            // of the last breakpoint in a bin: from it to the bin's end
     const uint16_t* bin;    // the breakpoint's bin
+    const uint32_t* narrow; // breakpoints behind elements without width
+    const uint16_t* owner;  // the breakpoint's PCF
+    const float* fwd;       // distances only, with the PCFs' norms
+    const float* norm;
   };
 
   struct L2BackwardPlan
@@ -50,7 +55,7 @@ namespace sbg
     uint32_t bins = 0, rows = 0;
     uint64_t k = 0, width = 0;  // rows of the table; rows of the gradient at a time
     size_t bytes = 0;
-    size_t record = 0, edges = 0, counts = 0, starts = 0, next = 0, centre = 0, norm = 0, keys = 0, event = 0, pcf = 0, owner = 0,
+    size_t record = 0, edges = 0, counts = 0, starts = 0, next = 0, centre = 0, norm = 0, narrow = 0, keys = 0, event = 0, pcf = 0, owner = 0,
            point = 0, place = 0, area = 0, rest = 0, bin = 0, table = 0, wt = 0, product = 0;
   };
 

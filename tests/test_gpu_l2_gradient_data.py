@@ -147,3 +147,24 @@ def test_each_value_gradient_against_its_own_terms(kind, n, lo, hi):
     last[off[1:] - 1] = True
     err = ((got[:, 1].double() - want[:, 1]).abs() / scale)[~last]
     assert float(err.max()) <= 4 * (256 + n / 256 + 64 + 14) * 2.0 ** -24, float(err.max())
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("each", [1, 3])
+def test_elements_without_width_at_shared_times(kind, each):
+    """Times on a grid, where other PCFs have breakpoints at the same time as
+    an element without width; one such element in a PCF, or three, of which
+    there are more than PCFs."""
+    import torch
+    n, points = 1000, 120
+    pts, off = _data(n, points, points, seed=11)
+    rng = np.random.default_rng(12)
+    t = np.concatenate([np.r_[0.0, np.sort(rng.choice(2000, points - 1, replace=False) + 1) / 16] for _ in range(n)])
+    pts[:, 0] = torch.from_numpy(t.astype(np.float32)).cuda()
+    for e in range(each):
+        k = off[:-1] + 20 + 30 * e
+        pts[k, 0] = pts[k - 1, 0]
+    if each == 3:
+        pts[off[:-1:4] + 50 + 1, 0] = pts[off[:-1:4] + 50, 0]  # three breakpoints at one time
+    w = _weights(n, kind, 13)
+    _near(_run(pts, off, kind, w)[1], _run(pts.double(), off, kind, w.double())[1])
