@@ -108,7 +108,11 @@ namespace sbg
     // Bin edges: quantiles of a sample of the breakpoint times, sorted in
     // shared memory by one CTA; edge 0 is time 0, edge `bins` the last time.
     // Only points that the offsets cover: what stands behind them may be
-    // anything, and a NaN would leave the edges out of order.
+    // anything, and a NaN would leave the edges out of order.  One point out
+    // of each of 8192 equal stretches, at a fraction that runs through [0, 1)
+    // in steps of the golden ratio: at a fixed place, PCFs of one length are
+    // sampled at the same few of their breakpoints (N = 4096, L = 264: two),
+    // whose quantiles leave bins too full to sort.
     __global__ void __launch_bounds__(1024) l2_edges_kernel(const float* __restrict__ pts,
                                                             const uint64_t* __restrict__ off, uint64_t n,
                                                             const L2Record* __restrict__ rec, uint32_t bins,
@@ -117,7 +121,7 @@ namespace sbg
       __shared__ float s[SAMPLES];
       if (rec->bad) return;
       const uint64_t o = off[0], covered = off[n] - o;
-      for (uint32_t q = threadIdx.x; q < SAMPLES; q += 1024) s[q] = pts[2 * (o + q * covered / SAMPLES)];
+      for (uint32_t q = threadIdx.x; q < SAMPLES; q += 1024) s[q] = pts[2 * (o + (q * covered + ((uint64_t)(q * 0x9e3779b9u) * covered >> 32)) / SAMPLES)];
       // a stage at distance 32 or less stays within the 64 elements of a warp
       uint32_t before = 64;  // the loads cross warps
       for (uint32_t k = 2; k <= SAMPLES; k <<= 1)

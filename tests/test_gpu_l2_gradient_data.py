@@ -168,3 +168,15 @@ def test_elements_without_width_at_shared_times(kind, each):
         pts[off[:-1:4] + 50 + 1, 0] = pts[off[:-1:4] + 50, 0]  # three breakpoints at one time
     w = _weights(n, kind, 13)
     _near(_run(pts, off, kind, w)[1], _run(pts.double(), off, kind, w.double())[1])
+
+
+@pytest.mark.parametrize("n,points", [(4096, 128), (2048, 256), (1024, 1024)])
+def test_pcfs_of_one_length(n, points):
+    """Lengths that divide the stretches the edges are sampled from: the bins
+    stay even and the contraction runs, whose kernel gradients add nothing
+    atomically, so that a second run gives the same bits."""
+    pts, off = _data(n, points, points, seed=points)
+    w = _weights(n, "kernel", 5)
+    got = _run(pts, off, "kernel", w)[1]
+    assert bool((got == _run(pts, off, "kernel", w)[1]).all())
+    _near(got, _run(pts.double(), off, "kernel", w.double())[1])
