@@ -57,7 +57,8 @@ def set_tuning(warps: int = 0, row_chunk: int = 0, variant: int = 0, order: int 
     unified shared-memory load per step from a row replicated 16 times, and
     8, merge path with one pair per warp, which the planner never picks),
     PCF order (1 as given, 2 sorted by breakpoint count), output bytes per
-    pipeline band."""
+    pipeline band.  float64 L1, L2 and L2 kernel calls without a variant or
+    window cap run in fixed point, with at most 16 warps and 1024 rows."""
     nat.check(nat.lib().sbg_set_tuning(int(warps), int(row_chunk), int(variant), int(order), int(band_bytes)))
 
 
