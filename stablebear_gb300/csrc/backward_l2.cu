@@ -24,7 +24,7 @@
 // 2 bins FMAs and L^2 / bins list entries.  Nothing is added atomically, and
 // the sums are shorter.  N = 4096, L ~ U{16..512}, L2 kernel, forward and
 // backward: 14.4 -> 4.8 ms (the forward is 2.4 of it), error of the gradient
-// 8.5e-7 -> 3.0e-7; of each value's gradient against the sum of its own
+// 8.5e-7 -> 2.5e-7; of each value's gradient against the sum of its own
 // |terms|, N = 1000, segments from a millionth of a time unit on: rms 1.2e-8 to
 // 1.4e-8 over the first three quarters of the time and 3e-8 to 1.4e-7 behind,
 // 2.1e-8 in the walk (with differences from the edge up to 20, rms 5e-2).
@@ -819,39 +819,60 @@ namespace sbg
         const float* hint = P.product + (i - P.r0) * 2 * P.bins + P.bins;
         const float sum = KERNEL ? 0.0f : s_sum[r];
         const float wii = KERNEL ? P.grad_out[i * (i + 1) / 2 + i] : 0.0f;
-        for (uint32_t k = lane; k < len; k += 32)
+        for (uint32_t k = lane; k + 1 < len; k += 32)
         {
           const float v = P.pts[2 * (o + k) + 1];
-          const float t0 = k ? P.pts[2 * (o + k)] : 0.0f;
-          const uint32_t b0 = k ? P.bin[o + k] : 0u;
-          const bool last = k + 1 == len;
-          const float t1 = last ? P.edges[P.bins] : P.pts[2 * (o + k + 1)];
-          const uint32_t b1 = last ? P.bins - 1 : P.bin[o + k + 1];
+          const float t0 = k ? P.pts[2 * (o + k)] : 0.0f, t1 = P.pts[2 * (o + k + 1)];
+          const uint32_t b0 = k ? P.bin[o + k] : 0u, b1 = P.bin[o + k + 1];
           // the part of the first bin, whole bins, the part of the last one
-          float H = 0.0f, own = 0.0f;
+          float H = P.area[o + k + 1], own = 0.0f;
           if (b0 == b1)
           {
-            H = !last ? P.area[o + k + 1] : k ? P.rest[o + k] : hint[b0];
             if (!KERNEL) own = (v - P.centre[b0]) * (t1 - t0);
           }
           else
           {
-            H = k ? P.rest[o + k] : hint[b0];
+            float whole = k ? P.rest[o + k] : hint[b0];
             if (!KERNEL) own = (v - P.centre[b0]) * (P.edges[b0 + 1] - t0);
             for (uint32_t b = b0 + 1; b < b1; ++b)
             {
-              H += hint[b];
+              whole += hint[b];
               if (!KERNEL) own = fmaf(v - P.centre[b], P.edges[b + 1] - P.edges[b], own);
             }
-            H += last ? hint[b1] : P.area[o + k + 1];
+            H += whole;
             if (!KERNEL) own = fmaf(v - P.centre[b1], t1 - P.edges[b1], own);
           }
           float dv = KERNEL ? H : fmaf(own, sum, -H);
-          // the kernel's diagonal; a last element, 0, ends nowhere
-          if (KERNEL && !last) dv = fmaf(wii, 2.0f * (v * (t1 - t0)), dv);
+          if (KERNEL) dv = fmaf(wii, 2.0f * (v * (t1 - t0)), dv);  // the kernel's diagonal
           P.grad[2 * (o + k) + 1] = dv;
           if (k == 0) P.grad[2 * o] = 0.0f;
           lost |= !isfinite(dv);
+        }
+        // The last element, 0 up to the end of time: of the shorter PCFs most of
+        // the bins, by the whole warp.
+        {
+          const uint32_t k = len - 1, b0 = k ? P.bin[o + k] : 0u;
+          float H = 0.0f, own = 0.0f;
+          for (uint32_t b = b0 + 1 + lane; b < P.bins; b += 32)
+          {
+            H += hint[b];
+            if (!KERNEL) own = fmaf(-P.centre[b], P.edges[b + 1] - P.edges[b], own);
+          }
+#pragma unroll
+          for (int d = 16; d > 0; d >>= 1)
+          {
+            H += __shfl_xor_sync(FULL, H, d);
+            if (!KERNEL) own += __shfl_xor_sync(FULL, own, d);
+          }
+          if (lane == 0)
+          {
+            H += k ? P.rest[o + k] : hint[b0];
+            if (!KERNEL) own = fmaf(-P.centre[b0], P.edges[b0 + 1] - (k ? P.pts[2 * (o + k)] : 0.0f), own);
+            const float dv = KERNEL ? H : fmaf(own, sum, -H);
+            P.grad[2 * (o + k) + 1] = dv;
+            if (k == 0) P.grad[2 * o] = 0.0f;
+            lost |= !isfinite(dv);
+          }
         }
       }
       if (__any_sync(FULL, lost) && lane == 0) atomicOr(&P.rec->bad_weights, 1u);
