@@ -373,12 +373,18 @@ namespace sbg
           tv += __shfl_xor_sync(FULL, tv, h);
           qv += __shfl_xor_sync(FULL, qv, h);
           ev += __shfl_xor_sync(FULL, ev, h);
-          vm = fmaxf(vm, __shfl_xor_sync(FULL, vm, h));
           area += __shfl_xor_sync(FULL, area, h);
-          end = fmaxf(end, __shfl_xor_sync(FULL, end, h));
-          lo = fminf(lo, __shfl_xor_sync(FULL, lo, h));
-          hi = fmaxf(hi, __shfl_xor_sync(FULL, hi, h));
         }
+        // floats >= 0 order as their bits; the others after this
+        auto order = [](float x) {
+          const int b = __float_as_int(x);
+          return b ^ ((b >> 31) & 0x7fffffff);
+        };
+        auto value_of = [](int b) { return __int_as_float(b ^ ((b >> 31) & 0x7fffffff)); };
+        vm = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(vm)));
+        end = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(end)));
+        lo = value_of(__reduce_min_sync(FULL, order(lo)));
+        hi = value_of(__reduce_max_sync(FULL, order(hi)));
         if (lane == 0)
         {
           times[o + count - 1] = f.kind == 1 ? ((T_END >> 31) << 32) | (T_END & 0x7fffffffull) : T_END;
